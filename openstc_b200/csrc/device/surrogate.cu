@@ -16,6 +16,7 @@
 
 #include "engine.hpp"
 #include "kernels_surrogate.cuh"
+#include "mlp_train.cuh"
 #include "openstc_b200.h"
 #include "surrogate.hpp"
 #include "tc_gemm.cuh"
@@ -93,17 +94,6 @@ __device__ inline double gauss(uint64_t &s) {
 
 __device__ inline uint16_t bf16(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
 __device__ inline float from_bf16(uint16_t v) { return __bfloat162float(__ushort_as_bfloat16(v)); }
-
-// GELU in its tanh form (the inference kernel evaluates the same form with
-// the hardware tanh)
-__device__ inline float gelu(float x) {
-  const float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
-  return 0.5f * x * (1.f + t);
-}
-__device__ inline float gelu_grad(float x) {
-  const float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
-}
 
 // ------------------------------------------------------------------ samples
 // T, p, Y[9], dt per sample: from the cells of a flow field (perturbed) or
@@ -215,132 +205,35 @@ __global__ void k_features(const double *states, const double *dy, int64_t n, No
 }
 
 // ---------------------------------------------------------------- training
-__global__ void k_gather(const uint16_t *x, const float *t, int64_t n_train, uint64_t seed, int batch, uint16_t *a0,
-                         uint16_t *a0t, float *tb) {
+// Rows of the batch into the first layer's operand image and the target
+// buffer: row i of the data (in order; rows past n are zero) or a random one
+// of its n rows.
+__global__ void k_gather(const uint16_t *x, const float *t, int64_t n, uint64_t seed, bool in_order, int batch,
+                         uint8_t *a0, float *tb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= batch) return;
-  const int64_t src = static_cast<int64_t>(mix64(seed ^ mix64(static_cast<uint64_t>(i) + 7)) % n_train);
-  for (int q = 0; q < kSurInPad; ++q) {
-    const uint16_t v = x[src * kSurInPad + q];
-    a0[static_cast<int64_t>(i) * kSurInPad + q] = v;
-    a0t[static_cast<int64_t>(q) * batch + i] = v;
-  }
-  for (int q = 0; q < kSurOutPad; ++q) tb[static_cast<int64_t>(i) * kSurOutPad + q] = t[src * kSurOutPad + q];
+  const int64_t src = in_order ? i : static_cast<int64_t>(mix64(seed ^ mix64(static_cast<uint64_t>(i) + 7)) % n);
+  const bool live = src < n;
+  const uint4 *xs = reinterpret_cast<const uint4 *>(x + src * kSurInPad);
+  uint8_t *img = a0 + static_cast<int64_t>(i / mlp::kTile) * mlp::kChunk;
+  for (int p = 0; p < 2; ++p)
+    *reinterpret_cast<uint4 *>(img + mlp::image_offset(mlp::kTile, i % mlp::kTile, 8 * p)) =
+        live ? xs[p] : make_uint4(0, 0, 0, 0);
+  if (!t) return;
+  const float4 *ts = reinterpret_cast<const float4 *>(t + src * kSurOutPad);
+  float4 *to = reinterpret_cast<float4 *>(tb + static_cast<int64_t>(i) * kSurOutPad);
+  for (int p = 0; p < kSurOutPad / 4; ++p) to[p] = live ? ts[p] : make_float4(0, 0, 0, 0);
 }
 
-// v = src (+ bias) [mode 0: linear; 1: store pre-activation, out = GELU;
-// 2: v = src * GELU'(zpre)]; writes v (FP32, optional), out (bf16 rows x d)
-// and its transpose (bf16 d x rows).  Tiles of 32 x 32 through shared memory.
-__global__ void k_act(const float *src, int rows, int d, const float *bias, const float *zpre, int mode, float *vout,
-                      uint16_t *out, uint16_t *outt) {
-  __shared__ uint16_t tile[32][34];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int rr = threadIdx.y; rr < 32; rr += blockDim.y) {
-    const int r = r0 + rr, c = c0 + threadIdx.x;
-    uint16_t o = 0;
-    if (r < rows && c < d) {
-      const int64_t idx = static_cast<int64_t>(r) * d + c;
-      float v = src[idx];
-      float a = v;
-      if (mode == 0) {
-        if (bias) v += bias[c];
-        a = v;
-      } else if (mode == 1) {
-        v += bias[c];
-        a = gelu(v);
-      } else {
-        v *= gelu_grad(zpre[idx]);
-        a = v;
-      }
-      if (vout) vout[idx] = v;
-      o = bf16(a);
-      out[idx] = o;
-    }
-    tile[rr][threadIdx.x] = o;
-  }
-  __syncthreads();
-  for (int cc = threadIdx.y; cc < 32; cc += blockDim.y) {
-    const int c = c0 + cc, r = r0 + threadIdx.x;
-    if (c < d && r < rows) outt[static_cast<int64_t>(c) * rows + r] = tile[threadIdx.x][cc];
-  }
-}
-
-// output layer: pred = z + b; loss += mean (pred - t)^2 over 9 outputs;
-// dz = 2 (pred - t) / (batch * 9) (padding columns zero)
-__global__ void k_out_grad(float *z, const float *b, const float *t, int batch, float *dz, double *loss) {
-  __shared__ double sh[256];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double l = 0;
-  if (i < batch) {
-    for (int q = 0; q < kSurOutPad; ++q) {
-      const int64_t idx = static_cast<int64_t>(i) * kSurOutPad + q;
-      float g = 0;
-      if (q < kSurOut) {
-        const float pred = z[idx] + b[q];
-        z[idx] = pred;
-        const float e = pred - t[idx];
-        l += static_cast<double>(e) * e;
-        g = 2.f * e / (static_cast<float>(batch) * kSurOut);
-      }
-      dz[idx] = g;
-    }
-  }
-  sh[threadIdx.x] = l;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) atomicAdd(loss, sh[0] / (static_cast<double>(batch) * kSurOut));
-}
-
-__global__ void k_colsum(const float *v, int rows, int d, float *out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
-  const int per = (rows + gridDim.y - 1) / gridDim.y;
-  const int r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
-  float s = 0;
-  for (int r = r0; r < r1; ++r) s += v[static_cast<int64_t>(r) * d + c];
-  atomicAdd(&out[c], s);
-}
-
-__global__ void k_transpose16(const uint16_t *in, int rows, int d, uint16_t *out) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= static_cast<int64_t>(rows) * d) return;
-  const int r = static_cast<int>(i / d), c = static_cast<int>(i % d);
-  out[static_cast<int64_t>(c) * rows + r] = in[i];
-}
-
-__global__ void k_reduce(const float *partial, int splits, int64_t count, float *out) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= count) return;
-  float s = 0;
-  for (int q = 0; q < splits; ++q) s += partial[q * count + i];
-  out[i] = s;
-}
-
-__global__ void k_adam(float *p, const float *g, float *m, float *v, int64_t n, float lr, float b1, float b2,
-                       float eps, float bc1, float bc2) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1 - b1) * gi, vi = b2 * v[i] + (1 - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-}
-
-// bf16 copies of a weight [dout x din]: row-major, transposed, and in the
-// tile order of the fused inference kernel (K chunks of 16 columns).
-__global__ void k_pack(const float *w, int dout, int din, uint16_t *wb, uint16_t *wbt, uint8_t *wp) {
-  // wp null: the training GEMMs' copies only
+// bf16 copies of a weight [dout x din]: the operand image of the training
+// kernels and the tile order of the fused inference kernel (K chunks of 16
+// columns).
+__global__ void k_pack(const float *w, int dout, int din, uint8_t *img, uint8_t *wp) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= static_cast<int64_t>(dout) * din) return;
   const int r = static_cast<int>(i / din), k = static_cast<int>(i % din);
   const uint16_t v = bf16(w[i]);
-  wb[i] = v;
-  wbt[static_cast<int64_t>(k) * dout + r] = v;
-  if (!wp) return;
+  *reinterpret_cast<uint16_t *>(img + mlp::image_offset(dout, r, k)) = v;
   const int bk = 16;
   const int c = k / bk, kk = k % bk;
   *reinterpret_cast<uint16_t *>(wp + static_cast<size_t>(c) * dout * bk * 2 + tc::tile_offset(r, kk, bk)) = v;
@@ -380,8 +273,7 @@ Surrogate::Surrogate(const DevParams &chem, const std::vector<int> &elem_comp, i
     vw_[l] = static_cast<float *>(alloc(nw * 4));
     mb_[l] = static_cast<float *>(alloc(dout_[l] * 4));
     vb_[l] = static_cast<float *>(alloc(dout_[l] * 4));
-    wb_[l] = static_cast<uint16_t *>(alloc(nw * 2));
-    wbt_[l] = static_cast<uint16_t *>(alloc(nw * 2));
+    wimg_[l] = static_cast<uint8_t *>(alloc(static_cast<size_t>(dout_[l]) * ((din_[l] + 63) / 64) * 128));
     wpack_[l] = static_cast<uint8_t *>(alloc(nw * 2));
     ck(cudaMemcpyAsync(w_[l], w.data(), nw * 4, cudaMemcpyHostToDevice, stream_), "upload weights");
     ck(cudaMemcpyAsync(b_[l], b.data(), dout_[l] * 4, cudaMemcpyHostToDevice, stream_), "upload bias");
@@ -407,6 +299,7 @@ Surrogate::Surrogate(const DevParams &chem, const std::vector<int> &elem_comp, i
 Surrogate::~Surrogate() {
   cudaSetDevice(device_);
   for (void *p : allocs_) cudaFree(p);
+  free_batch();
   cudaFree(states_);
   cudaFree(labels_);
   cudaFree(x_);
@@ -426,7 +319,7 @@ void Surrogate::upload_chem() {
 void Surrogate::pack() {
   for (int l = 0; l < kSurLayers; ++l) {
     const int64_t nw = static_cast<int64_t>(dout_[l]) * din_[l];
-    k_pack<<<(nw + 255) / 256, 256, 0, stream_>>>(w_[l], dout_[l], din_[l], wb_[l], wbt_[l], wpack_[l]);
+    k_pack<<<(nw + 255) / 256, 256, 0, stream_>>>(w_[l], dout_[l], din_[l], wimg_[l], wpack_[l]);
   }
   ck(cudaGetLastError(), "pack weights");
   packed_ = true;
@@ -510,90 +403,140 @@ void Surrogate::generate(int64_t n, uint64_t seed, const DevBlock *field, double
   ck(cudaStreamSynchronize(stream_), "generate");
 }
 
-void Surrogate::ensure_batch(int batch) {
-  if (batch == batch_) return;
-  if (batch % 128) throw std::runtime_error("batch must be a multiple of 128");
+void Surrogate::free_batch() {
   auto free_ = [](auto *&p) {
     cudaFree(p);
     p = nullptr;
   };
   for (int l = 0; l < kSurLayers; ++l) {
     free_(a_[l]);
-    free_(at_[l]);
-    free_(z_[l]);
+    free_(dz_[l]);
+    free_(part_[l]);
+    free_(colsum_[l]);
   }
-  free_(dz_);
-  free_(dzt_);
-  free_(dzf_);
-  free_(da_);
-  free_(partial_);
-  free_(gw_);
-  free_(gb_);
+  for (auto &z : z_) free_(z);
+  free_(xb_);
   free_(tb_);
-  const size_t B = static_cast<size_t>(batch);
+  free_(pred_);
+  free_(loss_part_);
+  free_(grad_);
+  batch_ = 0;
+}
+
+void Surrogate::ensure_batch(int batch) {
+  if (batch == batch_) return;
+  if (batch % mlp::kTile) throw std::runtime_error("batch must be a multiple of 128");
+  free_batch();
+  const size_t B = static_cast<size_t>(batch), tiles = B / mlp::kTile;
+  const int halves = 2 * static_cast<int>(tiles), L = kSurLayers - 1;
+  size_t n_param = 0;
   for (int l = 0; l < kSurLayers; ++l) {
-    ck(cudaMalloc(&a_[l], B * din_[l] * 2), "act");
-    ck(cudaMalloc(&at_[l], B * din_[l] * 2), "act t");
-    ck(cudaMalloc(&z_[l], B * dout_[l] * 4), "z");
+    const bool thin = l == 0 || l == L;
+    splits_[l] = std::min(halves, thin ? mlp::kSplitThin : mlp::kSplitHidden);
+    ck(cudaMalloc(&a_[l], tiles * (l == 0 ? mlp::kChunk : mlp::kTileBytes)), "activations");
+    ck(cudaMalloc(&dz_[l], tiles * (l == L ? mlp::kChunk : mlp::kTileBytes)), "output gradients");
+    ck(cudaMalloc(&part_[l], static_cast<size_t>(splits_[l]) * kSurHidden * (thin ? 16 : kSurHidden) * 4), "partial");
+    ck(cudaMalloc(&colsum_[l], tiles * dout_[l] * 4), "column sums");
+    if (l < L) ck(cudaMalloc(&z_[l], B * kSurHidden * 4), "z");
+    n_param += static_cast<size_t>(dout_[l]) * din_[l] + dout_[l];
   }
-  ck(cudaMalloc(&dz_, B * kSurHidden * 2), "dz");
-  ck(cudaMalloc(&dzt_, B * kSurHidden * 2), "dzt");
-  ck(cudaMalloc(&dzf_, B * kSurHidden * 4), "dzf");
-  ck(cudaMalloc(&da_, B * kSurHidden * 4), "da");
-  ck(cudaMalloc(&partial_, 64ull * kSurHidden * kSurHidden * 4), "partial");
-  ck(cudaMalloc(&gw_, static_cast<size_t>(kSurHidden) * kSurHidden * 4), "gw");
-  ck(cudaMalloc(&gb_, kSurHidden * 4), "gb");
-  ck(cudaMalloc(&tb_, B * kSurOutPad * 4), "tb");
+  ck(cudaMalloc(&xb_, B * kSurInPad * 2), "features");
+  ck(cudaMalloc(&tb_, B * kSurOutPad * 4), "targets");
+  ck(cudaMalloc(&pred_, B * kSurOutPad * 4), "predictions");
+  ck(cudaMalloc(&loss_part_, tiles * sizeof(double)), "loss");
+  ck(cudaMalloc(&grad_, n_param * 4), "gradients");
+  auto smem = [](const void *fn, uint32_t bytes) {
+    ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)), "smem");
+  };
+  smem(reinterpret_cast<const void *>(mlp::k_layer<false, true>), mlp::kLayerSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_layer<false, false>), mlp::kLayerSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_layer<true, true>), mlp::kLayerSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_layer<true, false>), mlp::kLayerSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_out<true>), mlp::kOutSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_out<false>), mlp::kOutSmem);
+  smem(reinterpret_cast<const void *>(mlp::k_dw), mlp::kDwSmem);
   batch_ = batch;
 }
 
-// Forward pass of the batch in a_[0]: z_[l] = a_[l] W_l^T + b_l, a_[l+1] = GELU(z_[l]).
-void Surrogate::forward(int batch) {
-  for (int l = 0; l < kSurLayers; ++l) {
-    ck(tc_gemm(a_[l], din_[l], wb_[l], din_[l], z_[l], dout_[l], batch, dout_[l], din_[l], 1, err_, stream_),
-       "forward gemm");
-    if (l < kSurLayers - 1) {
-      const dim3 grid((dout_[l] + 31) / 32, (batch + 31) / 32);
-      k_act<<<grid, dim3(32, 8), 0, stream_>>>(z_[l], batch, dout_[l], b_[l], nullptr, 1, z_[l], a_[l + 1], at_[l + 1]);
-    }
+void Surrogate::gather(const uint16_t *x, const float *t, int64_t n, uint64_t seed, bool in_order) {
+  k_gather<<<(batch_ + 127) / 128, 128, 0, stream_>>>(x, t, n, seed, in_order, batch_, a_[0], tb_);
+  ck(cudaGetLastError(), "gather");
+}
+
+// The hidden layers of the batch in a_[0]: z = a_[l] W_l^T + b_l (kept for
+// the backward pass), a_[l + 1] = GELU(z).
+void Surrogate::forward(bool keep) {
+  const int tiles = batch_ / mlp::kTile;
+  for (int l = 0; l < kSurLayers - 1; ++l) {
+    auto *fn = l == 0 ? mlp::k_layer<false, true> : mlp::k_layer<false, false>;
+    fn<<<tiles, mlp::kThreads, mlp::kLayerSmem, stream_>>>(a_[l], wimg_[l], b_[l], keep ? z_[l] : nullptr, a_[l + 1],
+                                                          nullptr, err_);
   }
   ck(cudaGetLastError(), "forward");
 }
 
-double Surrogate::backward_and_step(int batch, double lr, int step) {
-  ck(cudaMemsetAsync(loss_, 0, sizeof(double), stream_), "loss");
+// The output layer: loss and output gradient of the batch's targets, or the
+// predictions.
+void Surrogate::output_layer(bool train) {
   const int L = kSurLayers - 1;
-  k_out_grad<<<(batch + 255) / 256, 256, 0, stream_>>>(z_[L], b_[L], tb_, batch, dzf_, loss_);
-  {
-    const dim3 grid((kSurOutPad + 31) / 32, (batch + 31) / 32);
-    k_act<<<grid, dim3(32, 8), 0, stream_>>>(dzf_, batch, kSurOutPad, nullptr, nullptr, 0, nullptr, dz_, dzt_);
+  auto *fn = train ? mlp::k_out<true> : mlp::k_out<false>;
+  fn<<<batch_ / mlp::kTile, mlp::kTile, mlp::kOutSmem, stream_>>>(a_[L], wimg_[L], b_[L], tb_, batch_, pred_, dz_[L],
+                                                                 colsum_[L], loss_part_, err_);
+  ck(cudaGetLastError(), "output layer");
+}
+
+// Output gradients of every layer down from dz_[L], then the partial weight
+// gradients of all layers.
+void Surrogate::backward() {
+  const int L = kSurLayers - 1;
+  for (int l = L; l > 0; --l) {
+    auto *fn = l == L ? mlp::k_layer<true, true> : mlp::k_layer<true, false>;
+    fn<<<batch_ / mlp::kTile, mlp::kThreads, mlp::kLayerSmem, stream_>>>(dz_[l], wimg_[l], nullptr, z_[l - 1], dz_[l - 1],
+                                                                        colsum_[l - 1], err_);
   }
-  ++adam_t_;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float bc1 = 1.f - std::pow(b1, static_cast<float>(adam_t_)), bc2 = 1.f - std::pow(b2, static_cast<float>(adam_t_));
-  const int splits = std::max(1, std::min(64, batch / 1024));
-  for (int l = L; l >= 0; --l) {
-    const int dout = dout_[l], din = din_[l];
-    // dW = dZ^T A  (K = batch, split-K)
-    ck(tc_gemm(dzt_, batch, at_[l], batch, partial_, din, dout, din, batch, splits, err_, stream_), "dW gemm");
-    const int64_t nw = static_cast<int64_t>(dout) * din;
-    k_reduce<<<(nw + 255) / 256, 256, 0, stream_>>>(partial_, splits, nw, gw_);
-    ck(cudaMemsetAsync(gb_, 0, dout * 4, stream_), "gb");
-    k_colsum<<<dim3((dout + 127) / 128, 64), 128, 0, stream_>>>(dzf_, batch, dout, gb_);
-    // dA = dZ W (B operand: W^T rows), then dZ of the layer below
-    if (l > 0) {
-      ck(tc_gemm(dz_, dout, wbt_[l], dout, da_, din, batch, din, dout, 1, err_, stream_), "dA gemm");
-      const dim3 grid((din + 31) / 32, (batch + 31) / 32);
-      k_act<<<grid, dim3(32, 8), 0, stream_>>>(da_, batch, din, nullptr, z_[l - 1], 2, dzf_, dz_, dzt_);
-    }
-    k_adam<<<(nw + 255) / 256, 256, 0, stream_>>>(w_[l], gw_, mw_[l], vw_[l], nw, static_cast<float>(lr), b1, b2,
-                                                 1e-8f, bc1, bc2);
-    k_adam<<<(dout + 255) / 256, 256, 0, stream_>>>(b_[l], gb_, mb_[l], vb_[l], dout, static_cast<float>(lr), b1, b2,
-                                                   1e-8f, bc1, bc2);
+  mlp::DwArgs a{};
+  int grid = 0;
+  for (int l = 0; l < kSurLayers; ++l) {
+    a.p[l] = l == L ? a_[l] : dz_[l];
+    a.q[l] = l == L ? dz_[l] : a_[l];
+    a.part[l] = part_[l];
+    a.splits[l] = splits_[l];
+    grid += splits_[l];
   }
+  a.halves = 2 * (batch_ / mlp::kTile);
+  mlp::k_dw<<<grid, mlp::kThreads, mlp::kDwSmem, stream_>>>(a, err_);
   ck(cudaGetLastError(), "backward");
-  (void)step;
-  return 0;  // the loss accumulates in loss_ on the device
+}
+
+// Sums the partial gradients and the loss, and stores the gradients (grad) or
+// takes the Adam step with them.
+void Surrogate::reduce(float *grad, double lr, double *loss) {
+  mlp::StepArgs a{};
+  for (int l = 0; l < kSurLayers; ++l) {
+    a.w[l] = w_[l];
+    a.b[l] = b_[l];
+    a.mw[l] = mw_[l];
+    a.vw[l] = vw_[l];
+    a.mb[l] = mb_[l];
+    a.vb[l] = vb_[l];
+    a.img[l] = wimg_[l];
+    a.part[l] = part_[l];
+    a.colsum[l] = colsum_[l];
+    a.splits[l] = splits_[l];
+  }
+  a.tiles = batch_ / mlp::kTile;
+  a.batch = batch_;
+  a.loss_part = loss_part_;
+  a.loss = loss;
+  a.grad = grad;
+  a.lr = static_cast<float>(lr);
+  a.b1 = 0.9f;
+  a.b2 = 0.999f;
+  a.eps = 1e-8f;
+  a.bc1 = 1.f - std::pow(a.b1, static_cast<float>(adam_t_));
+  a.bc2 = 1.f - std::pow(a.b2, static_cast<float>(adam_t_));
+  mlp::k_step<<<mlp::kStepBlocks, dim3(32, 8), 0, stream_>>>(a);
+  ck(cudaGetLastError(), "gradient step");
 }
 
 double Surrogate::train(int steps, int batch, double lr, int64_t n_train, float *losses) {
@@ -606,19 +549,15 @@ double Surrogate::train(int steps, int batch, double lr, int64_t n_train, float 
   DevTemp<double> dloss_buf(static_cast<size_t>(std::max(1, steps)), "cudaMalloc losses");
   double *dloss = dloss_buf.p;
   for (int s = 0; s < steps; ++s) {
-    k_gather<<<(batch + 255) / 256, 256, 0, stream_>>>(x_, t_, n_train, mix64(seed_ + 0x5151 * (adam_t_ + 1)), batch,
-                                                       a_[0], at_[0], tb_);
-    forward(batch);
+    gather(x_, t_, n_train, mix64(seed_ + 0x5151 * (adam_t_ + 1)), false);
+    forward(true);
+    output_layer(true);
+    backward();
     const double cosine = 0.5 * (1 + std::cos(3.141592653589793 * s / std::max(1, steps)));
     // schedule: cosine decay to 5 % of lr
     const double lr_s = lr * (0.05 + 0.95 * cosine);
-    backward_and_step(batch, lr_s, s);
-    ck(cudaMemcpyAsync(dloss + s, loss_, sizeof(double), cudaMemcpyDeviceToDevice, stream_), "loss copy");
-    // new bf16 weights for the next step's GEMMs (the inference copy once, below)
-    for (int l = 0; l < kSurLayers; ++l) {
-      const int64_t nw = static_cast<int64_t>(dout_[l]) * din_[l];
-      k_pack<<<(nw + 255) / 256, 256, 0, stream_>>>(w_[l], dout_[l], din_[l], wb_[l], wbt_[l], nullptr);
-    }
+    ++adam_t_;
+    reduce(nullptr, lr_s, dloss + s);  // new bf16 images too; the inference copy once, below
   }
   pack();
   std::vector<double> hl(static_cast<size_t>(std::max(1, steps)), 0.0);
@@ -715,13 +654,11 @@ void Surrogate::predict_host(const double *states, int64_t n, double *dy, int *a
   int *acc = acc_buf.p;
   ck(cudaMemsetAsync(s, 0, static_cast<size_t>(batch) * kSurIn * 8, stream_), "predict memset");
   ck(cudaMemcpyAsync(s, states, n * kSurIn * 8, cudaMemcpyHostToDevice, stream_), "predict upload");
-  features(s, n, a_[0], nullptr, nullptr);
-  ck(cudaMemsetAsync(a_[0] + n * kSurInPad, 0, (batch - n) * kSurInPad * 2, stream_), "pad rows");
-  forward(batch);
-  const int L = kSurLayers - 1;
-  k_act<<<dim3(1, (batch + 31) / 32), dim3(32, 8), 0, stream_>>>(z_[L], batch, kSurOutPad, b_[L], nullptr, 0, z_[L],
-                                                                   dz_, dzt_);
-  k_decode<<<(n + 255) / 256, 256, 0, stream_>>>(z_[L], s, n, device_params(), d, acc);
+  features(s, n, xb_, nullptr, nullptr);
+  gather(xb_, nullptr, n, 0, true);
+  forward(false);
+  output_layer(false);
+  k_decode<<<(n + 255) / 256, 256, 0, stream_>>>(pred_, s, n, device_params(), d, acc);
   ck(cudaGetLastError(), "predict");
   ck(cudaMemcpyAsync(dy, d, n * NS * 8, cudaMemcpyDeviceToHost, stream_), "predict download");
   ck(cudaMemcpyAsync(accepted, acc, n * sizeof(int), cudaMemcpyDeviceToHost, stream_), "predict download");
@@ -737,33 +674,20 @@ double Surrogate::grad_host(const double *states, const double *dy, int64_t n, s
   double *s = s_buf.p, *d = d_buf.p;
   ck(cudaMemcpyAsync(s, states, n * kSurIn * 8, cudaMemcpyHostToDevice, stream_), "grad upload");
   ck(cudaMemcpyAsync(d, dy, n * NS * 8, cudaMemcpyHostToDevice, stream_), "grad upload");
-  features(s, n, a_[0], tb_, d);
-  k_transpose16<<<(n * kSurInPad + 255) / 256, 256, 0, stream_>>>(a_[0], batch, kSurInPad, at_[0]);
-  forward(batch);
-  // the backward pass of training without the Adam update, one layer at a time
+  features(s, n, xb_, tb_, d);
+  gather(xb_, nullptr, n, 0, true);
+  forward(true);
+  output_layer(true);
+  backward();
+  reduce(grad_, 0.0, loss_);
   grads.assign(2 * kSurLayers, {});
-  ck(cudaMemsetAsync(loss_, 0, sizeof(double), stream_), "loss");
-  const int L = kSurLayers - 1;
-  k_out_grad<<<(batch + 255) / 256, 256, 0, stream_>>>(z_[L], b_[L], tb_, batch, dzf_, loss_);
-  k_act<<<dim3(1, (batch + 31) / 32), dim3(32, 8), 0, stream_>>>(dzf_, batch, kSurOutPad, nullptr, nullptr, 0, nullptr,
-                                                                   dz_, dzt_);
-  const int splits = std::max(1, std::min(64, batch / 1024));
-  for (int l = L; l >= 0; --l) {
-    const int dout = dout_[l], din = din_[l];
-    ck(tc_gemm(dzt_, batch, at_[l], batch, partial_, din, dout, din, batch, splits, err_, stream_), "dW gemm");
-    const int64_t nw = static_cast<int64_t>(dout) * din;
-    k_reduce<<<(nw + 255) / 256, 256, 0, stream_>>>(partial_, splits, nw, gw_);
-    ck(cudaMemsetAsync(gb_, 0, dout * 4, stream_), "gb");
-    k_colsum<<<dim3((dout + 127) / 128, 64), 128, 0, stream_>>>(dzf_, batch, dout, gb_);
-    grads[2 * l].resize(nw);
-    grads[2 * l + 1].resize(dout);
-    ck(cudaMemcpyAsync(grads[2 * l].data(), gw_, nw * 4, cudaMemcpyDeviceToHost, stream_), "grad copy");
-    ck(cudaMemcpyAsync(grads[2 * l + 1].data(), gb_, dout * 4, cudaMemcpyDeviceToHost, stream_), "grad copy");
-    ck(cudaStreamSynchronize(stream_), "grad");
-    if (l > 0) {
-      ck(tc_gemm(dz_, dout, wbt_[l], dout, da_, din, batch, din, dout, 1, err_, stream_), "dA gemm");
-      const dim3 grid((din + 31) / 32, (batch + 31) / 32);
-      k_act<<<grid, dim3(32, 8), 0, stream_>>>(da_, batch, din, nullptr, z_[l - 1], 2, dzf_, dz_, dzt_);
+  size_t off = 0;
+  for (int l = 0; l < kSurLayers; ++l) {
+    grads[2 * l].resize(static_cast<size_t>(dout_[l]) * din_[l]);
+    grads[2 * l + 1].resize(dout_[l]);
+    for (int q = 2 * l; q < 2 * l + 2; ++q) {
+      ck(cudaMemcpyAsync(grads[q].data(), grad_ + off, grads[q].size() * 4, cudaMemcpyDeviceToHost, stream_), "grad copy");
+      off += grads[q].size();
     }
   }
   double loss = 0;

@@ -108,9 +108,13 @@ class Surrogate {
   SurrogateGate gate;
 
  private:
+  void free_batch();
   void ensure_batch(int batch);
-  void forward(int batch);
-  double backward_and_step(int batch, double lr, int step);
+  void gather(const uint16_t *x, const float *t, int64_t n, uint64_t seed, bool in_order);
+  void forward(bool keep);
+  void output_layer(bool train);
+  void backward();
+  void reduce(float *grad, double lr, double *loss);
   void pack();
   void upload_chem();
   void features(const double *states_dev, int64_t n, uint16_t *x_dev, float *t_dev, const double *dy_dev);
@@ -132,15 +136,18 @@ class Surrogate {
   int din_[kSurLayers], dout_[kSurLayers];
   float *w_[kSurLayers] = {}, *b_[kSurLayers] = {};
   float *mw_[kSurLayers] = {}, *vw_[kSurLayers] = {}, *mb_[kSurLayers] = {}, *vb_[kSurLayers] = {};
-  uint16_t *wb_[kSurLayers] = {}, *wbt_[kSurLayers] = {};
-  uint8_t *wpack_[kSurLayers] = {};
-  // batch work space
+  uint8_t *wimg_[kSurLayers] = {};   // bf16, the operand images of mlp_train.cuh
+  uint8_t *wpack_[kSurLayers] = {};  // bf16, the fused inference kernel's tile order
+  // batch work space: operand images of each layer's input and output
+  // gradient, FP32 pre-activations of the hidden layers, partial sums
   int batch_ = 0;
-  uint16_t *a_[kSurLayers] = {}, *at_[kSurLayers] = {};  // activations (input of layer l) and transposes
-  float *z_[kSurLayers] = {};                              // pre-activations of layer l
-  uint16_t *dz_ = nullptr, *dzt_ = nullptr;
-  float *dzf_ = nullptr, *da_ = nullptr, *partial_ = nullptr, *gw_ = nullptr, *gb_ = nullptr;
-  float *tb_ = nullptr;  // batch targets
+  uint8_t *a_[kSurLayers] = {}, *dz_[kSurLayers] = {};
+  float *z_[kSurLayers - 1] = {}, *part_[kSurLayers] = {}, *colsum_[kSurLayers] = {};
+  int splits_[kSurLayers] = {};
+  uint16_t *xb_ = nullptr;  // batch x 16 features (host samples)
+  float *tb_ = nullptr, *pred_ = nullptr;  // batch x 16 targets, predictions
+  double *loss_part_ = nullptr;
+  float *grad_ = nullptr;  // every gradient, in the flat parameter order
   double *loss_ = nullptr;
   int *err_ = nullptr;
   SurrogateDev dev_{};

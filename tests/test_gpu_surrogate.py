@@ -78,6 +78,33 @@ def test_gradients_match_oracle(drv):
             assert rel < 2e-3, (l, n, rel)
 
 
+@pytest.mark.parametrize("n", [128, 384, 128 * 37])
+def test_gradients_at_the_edges_of_the_splits(drv, n):
+    """One tile of 128 rows (fewer half tiles than weight-gradient splits), a
+    few, and a count that leaves the last splits short or empty: the same bound
+    as test_gradients_match_oracle (BF16 operands, FP32 sums; 4e-3 for fewer
+    rows, whose rounding averages over less)."""
+    sur = ostc.Surrogate(drv, seed=6)
+    sur.generate(4096, seed=3)
+    st = random_states(n, 13)
+    dy = sur.label(st)
+    loss, g = sur.gradients(st, dy)
+    mu, sig, c, sc = sur.normalisation()
+    x = mlp_oracle.features(st, mu, sig)
+    t = (np.arcsinh(dy / (st[:, 2:11] + 1e-10) / c.astype(np.float64)) / sc.astype(np.float64)).astype(np.float32)
+    loss_ref, g_ref = mlp_oracle.loss_and_grads(sur.params(), x, t.astype(np.float64))
+    assert abs(loss - loss_ref) <= 1e-4 * abs(loss_ref)
+    off = 0
+    for l in range(5):
+        for m in (mlp_oracle.DIMS[l] * mlp_oracle.DIMS[l + 1], mlp_oracle.DIMS[l + 1]):
+            a, b = g[off:off + m], g_ref[off:off + m]
+            off += m
+            assert np.linalg.norm(a - b) < 4e-3 * np.linalg.norm(b), (l, m)
+    # the same batch again: every sum has a fixed order
+    loss2, g2 = sur.gradients(st, dy)
+    assert loss2 == loss and np.array_equal(g, g2)
+
+
 def test_training_learns_and_gate(drv, tmp_path):
     sur = ostc.Surrogate(drv, seed=7)
     n = 1 << 19
