@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <stdexcept>
@@ -625,8 +626,7 @@ class EngineT final : public Engine {
   }
 
   // the tiles of direction pass d of the FP32-bulk flux (dir_tile_counts)
-  Tiles make_dir_tiles(int d) const {
-    const int march = kFluxVariant[flux_variant_].march;
+  Tiles make_dir_tiles(int d, int march) const {
     return build_tiles([d, march](const DevBlock &B, int &ntx, int &nty) {
       int n2 = 0;
       dir_tile_counts(d, march, B.mx, B.my, B.mz, ntx, nty, n2);
@@ -634,13 +634,80 @@ class EngineT final : public Engine {
     });
   }
 
-  // columns of kTX x kTY cells over kFluxKC planes (the k-marching flux kernel)
-  Tiles make_col_tiles() const {
-    return build_tiles([](const DevBlock &B, int &ntx, int &nty) {
+  // columns of kTX x kTY cells over kc planes (the k-marching flux kernel)
+  Tiles make_col_tiles(int kc) const {
+    return build_tiles([kc](const DevBlock &B, int &ntx, int &nty) {
       ntx = (B.mx + kTX - 1) / kTX;
       nty = (B.my + kTY - 1) / kTY;
-      return ntx * nty * ((B.mz + kFluxKC - 1) / kFluxKC);
+      return ntx * nty * ((B.mz + kc - 1) / kc);
     });
+  }
+
+  // rows of 32 cells (k_flux_row)
+  Tiles make_row_tiles() const {
+    return build_tiles([](const DevBlock &B, int &ntx, int &nty) {
+      ntx = (B.mx + 31) / 32;
+      nty = B.my;
+      return ntx * nty * B.mz;
+    });
+  }
+
+  // The time of a flux launch in units of one face evaluation on an idle SM:
+  // a thread evaluates `serial` faces one after another, which take up to 1 + a
+  // times as long once every slot (SMs x resident CTAs) is taken, and waves of
+  // CTAs follow each other (a wave's end overlaps the next one by about half).
+  static double flux_cost(double serial, int ctas, int slots, double a) {
+    const double w = static_cast<double>(ctas) / slots;
+    return serial * (1 + a * std::min(1.0, w)) * (w <= 1 ? 1.0 : 0.5 * (w + std::ceil(w)));
+  }
+
+  // How the flux kernels cut the grid.  Long columns or marches evaluate the
+  // fewest faces, short ones keep the SMs of a small grid busy; the constants
+  // are from event times on one B200.  FP64 (reacting layer, in us):
+  //   24 x 16 x 8:    8 / 4 / 2 / 1 planes 652 / 344 / 190 / 112, rows 24
+  //   45 x 37 x 21:                        707 / 381 / 225 / 240, rows 217
+  //   96 x 64 x 32:                        909 / 872 / 724 / 768, rows 868
+  //   160 x 96 x 64:                     3432 / 3291 / 3328 / 3537, rows 4199
+  // laminar ramp (columns, rows): 128 x 64 21, 11; 256 x 128 21, 25.
+  // FP32-bulk, y pass (march 8 / 4 / 2 / 1):
+  //   24 x 16 x 8: 153 / 88 / 54 / 39     96 x 64 x 32: 222 / 141 / 102 / 131
+  //   160 x 96 x 64: 336 / 364 / 412 / 457
+  void make_flux_tiles() {
+    if constexpr (C::mixed) {
+      const FluxVariant v = kFluxVariant[flux_variant_];
+      dir_tiles_[0] = make_dir_tiles(0, 1);
+      for (int d = 1; d < 3; ++d) {
+        double best = 0;
+        for (int m = v.march; m >= 1; m /= 2) {
+          const Tiles t = make_dir_tiles(d, m);
+          const double cost = flux_cost(m + 1, t.begin[t.nblk], num_sms_ * v.min_blocks, 1.25);
+          if (m < v.march && cost >= best) continue;
+          best = cost;
+          march_[d] = m;
+          dir_tiles_[d] = t;
+        }
+      }
+    } else {
+      bool three_d = false;
+      for (const auto &B : blocks_) three_d = three_d || B.mz > 1;
+      double best = 0;
+      for (int kc = three_d ? kFluxKC : 1; kc >= 1; kc /= 2) {
+        const Tiles t = make_col_tiles(kc);
+        const double cost = flux_cost(three_d ? 6 * kc + 2 : 4, t.begin[t.nblk], 2 * num_sms_, 0.35);
+        if (best > 0 && cost >= best) continue;
+        best = cost;
+        col_kc_ = kc;
+        col_tiles_ = t;
+      }
+      const Tiles t = make_row_tiles();
+      const double cost =
+          flux_cost(1.5, t.begin[t.nblk], (C::mix == 0 ? 2 : 1) * num_sms_, 0) + (three_d ? 0.0 : 0.9);
+      row_warps_ = 0;
+      if (cost < best) {
+        row_warps_ = 2 * (three_d ? kRowFaces : kRowFaces - 2);
+        col_tiles_ = t;
+      }
+    }
   }
 
   Tiles make_tiles(int halo) const {
@@ -657,8 +724,7 @@ class EngineT final : public Engine {
     tiles0_ = make_tiles(0);
     tiles1_ = make_tiles(1);
     tilesg_ = make_tiles(setup_.ngg);
-    col_tiles_ = make_col_tiles();
-    for (int d = 0; d < 3; ++d) dir_tiles_[d] = make_dir_tiles(d);
+    make_flux_tiles();
   }
 
   static dim3 grid(const Tiles &t) { return dim3(static_cast<unsigned>(t.begin[t.nblk])); }
@@ -693,27 +759,29 @@ class EngineT final : public Engine {
         k_pack32<C><<<pack_grid(b), 256, 0, stream_>>>(d_blocks_, b);
       mark("pack32");
       switch (flux_variant_) {
-        case 0: launch_flux_passes<kFluxVariant[0].min_blocks, kFluxVariant[0].march>(); break;
-        case 1: launch_flux_passes<kFluxVariant[1].min_blocks, kFluxVariant[1].march>(); break;
-        case 2: launch_flux_passes<kFluxVariant[2].min_blocks, kFluxVariant[2].march>(); break;
-        default: launch_flux_passes<kFluxVariant[3].min_blocks, kFluxVariant[3].march>(); break;
+        case 0: launch_flux_passes<kFluxVariant[0].min_blocks>(); break;
+        case 1: launch_flux_passes<kFluxVariant[1].min_blocks>(); break;
+        case 2: launch_flux_passes<kFluxVariant[2].min_blocks>(); break;
+        default: launch_flux_passes<kFluxVariant[3].min_blocks>(); break;
       }
     } else if (flux_variant_ == 1) {
       // the per-cell form: each face evaluated by both of its cells, no barriers
       k_flux<C><<<grid(tiles0_), block3(), flux_smem_, stream_>>>(d_blocks_, tiles0_);
+    } else if (row_warps_ > 0) {
+      k_flux_row<C><<<grid(col_tiles_), dim3(32, row_warps_), 0, stream_>>>(d_blocks_, col_tiles_);
     } else {
-      k_flux_col<C><<<grid(col_tiles_), kFluxThreads, col_smem_, stream_>>>(d_blocks_, col_tiles_);
+      k_flux_col<C><<<grid(col_tiles_), kFluxThreads, col_smem_, stream_>>>(d_blocks_, col_tiles_, col_kc_);
     }
   }
 
-  template <int MINB, int MARCH>
+  template <int MINB>
   void launch_flux_passes() {
     k_flux_x<C, MINB><<<grid(dir_tiles_[0]), kCta, 0, stream_>>>(d_blocks_, dir_tiles_[0]);
     mark("flux_x");
-    k_flux_march<C, 1, MINB, MARCH><<<grid(dir_tiles_[1]), kCta, 0, stream_>>>(d_blocks_, dir_tiles_[1]);
+    k_flux_march<C, 1, MINB><<<grid(dir_tiles_[1]), kCta, 0, stream_>>>(d_blocks_, dir_tiles_[1], march_[1]);
     mark("flux_y");
     if (setup_.params.dim == 3) {
-      k_flux_march<C, 2, MINB, MARCH><<<grid(dir_tiles_[2]), kCta, 0, stream_>>>(d_blocks_, dir_tiles_[2]);
+      k_flux_march<C, 2, MINB><<<grid(dir_tiles_[2]), kCta, 0, stream_>>>(d_blocks_, dir_tiles_[2], march_[2]);
       mark("flux_z");
     }
   }
@@ -1131,6 +1199,9 @@ class EngineT final : public Engine {
   Tiles tiles0_, tiles1_, tilesg_, col_tiles_, dir_tiles_[3];
   std::vector<int> order_;  // the blocks' schedule in every tile table (empty: block order)
   int flux_variant_ = 0;    // kFluxVariant entry of the FP32-bulk flux passes
+  int march_[3] = {1, 1, 1};  // cells a thread of the y / z pass marches over
+  int col_kc_ = kFluxKC;      // planes of a column (k_flux_col) ...
+  int row_warps_ = 0;         // ... or, when positive, the warps of a row (k_flux_row)
   WallGrid wall_grid_{};    // the bucket grid of the wall points (start null: brute force)
   size_t source_smem_ = 0, flux_smem_ = 0, col_smem_ = 0, dq0_smem_ = 0;
   int final_dq_ = 0;

@@ -683,14 +683,14 @@ __device__ __forceinline__ void local_time_step_s(const DevBlock &B, const Src &
 //   x: a warp holds 32 consecutive faces of one row (i - 1/2 + lane) and
 //      gives 31 cells their difference, the left face coming from the lane
 //      below by a shuffle; a CTA covers 4 rows (j).
-//   y, z: each thread marches kMarch cells along d, carrying the lower face
+//   y, z: each thread marches over some cells along d, carrying the lower face
 //      from one cell to the next; lanes run along i, the CTA's 4 warps over
 //      the remaining index (k for y, j for z).
 constexpr int kXSeg = 31;  // cells per warp of the x pass
 // The variants of the passes an autotuner chooses from: resident CTAs per
 // SM the register allocator is asked to allow (8 caps a thread at 64
 // registers, ~400 B of spills) and the cells a thread of the y / z pass
-// marches over.  Measured at 384x192x64 with a march of 8, the three passes
+// marches over at most (fewer where the grid would leave SMs idle).  Measured at 384x192x64 with a march of 8, the three passes
 // take 5.7 ms at 4 CTAs per SM, 5.0 at 6, 4.8 at 7, 4.4 at 8.  Every variant
 // computes the same values.
 struct FluxVariant {
@@ -701,8 +701,8 @@ constexpr FluxVariant kFluxVariant[kFluxVariants] = {{8, 8}, {8, 16}, {6, 8}, {4
 
 // Tiles of pass d over every block: (x) i-segments x row groups x k,
 // (y) i-groups x k-groups x j-segments, (z) i-groups x j-groups x k-segments
-// of kMarch cells.
-inline void dir_tile_counts(int d, int kMarch, int mx, int my, int mz, int &n0, int &n1, int &n2) {
+// of `march` cells.
+inline void dir_tile_counts(int d, int march, int mx, int my, int mz, int &n0, int &n1, int &n2) {
   if (d == 0) {
     n0 = (mx + kXSeg - 1) / kXSeg;
     n1 = (my + kTY - 1) / kTY;
@@ -710,11 +710,11 @@ inline void dir_tile_counts(int d, int kMarch, int mx, int my, int mz, int &n0, 
   } else if (d == 1) {
     n0 = (mx + kTX - 1) / kTX;
     n1 = (mz + kTY - 1) / kTY;
-    n2 = (my + kMarch - 1) / kMarch;
+    n2 = (my + march - 1) / march;
   } else {
     n0 = (mx + kTX - 1) / kTX;
     n1 = (my + kTY - 1) / kTY;
-    n2 = (mz + kMarch - 1) / kMarch;
+    n2 = (mz + march - 1) / march;
   }
 }
 
@@ -819,8 +819,8 @@ __global__ void __launch_bounds__(kCta, MINB) k_flux_x(const DevBlock *__restric
   if (cell) local_time_step_s<C>(B, fp32::Src32<C>{B.f32, B.G.size}, f, j, k, B.G.at(f, j, k), nd);
 }
 
-template <class C, int D, int MINB, int kMarch>
-__global__ void __launch_bounds__(kCta, MINB) k_flux_march(const DevBlock *__restrict__ blks, Tiles T) {
+template <class C, int D, int MINB>
+__global__ void __launch_bounds__(kCta, MINB) k_flux_march(const DevBlock *__restrict__ blks, Tiles T, int march) {
   constexpr int NV = C::nv;
   static_assert(D == 1 || D == 2, "march passes run along y or z");
   int b, t0, t1, t2;
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(kCta, MINB) k_flux_march(const DevBlock *__res
   const int i = t0 * kTX + lane, o = t1 * kTY + warp;  // o: k for the y pass, j for the z pass
   if (i >= B.mx || o >= (D == 1 ? B.mz : B.my)) return;
   const int m = D == 1 ? B.my : B.mz;
-  const int c0 = t2 * kMarch, c1 = min(c0 + kMarch, m);
+  const int c0 = t2 * march, c1 = min(c0 + march, m);
   const int64_t s = D == 1 ? B.G.sx : B.G.sxy;
   const int64_t n0 = D == 1 ? B.G.at(i, c0, o) : B.G.at(i, o, c0);
   const int64_t sd = D == 1 ? B.D.sx : B.D.sxy;

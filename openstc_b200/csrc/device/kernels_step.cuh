@@ -198,11 +198,12 @@ __global__ void __launch_bounds__(kCta, OSTC_FLUX_MIN_BLOCKS) k_flux(const DevBl
 // a plane is the high-k face of the plane before (shared memory).  Each face
 // value is the one k_flux computes for it and the per-cell sums run in the
 // same order (dq -= f(+) - f(-) per direction, inviscid then viscous), so the
-// result is bit-identical.
-constexpr int kFluxKC = 8;                  // k planes per column
+// result is bit-identical.  The planes per column (kc, at most kFluxKC) are
+// chosen by the launch.
+constexpr int kFluxKC = 8;                  // k planes per column at most
 constexpr int kFluxThreads = kCta + 32;     // 4 compute warps + the minus-face warp
 
-__device__ __forceinline__ void col_tile(const Tiles &T, int &b, int &i0, int &j0, int &k0) {
+__device__ __forceinline__ void col_tile(const Tiles &T, int kc, int &b, int &i0, int &j0, int &k0) {
   int t = tile_of(T, blockIdx.x, b);
   const int tx = t % T.ntx[b];
   t /= T.ntx[b];
@@ -210,7 +211,7 @@ __device__ __forceinline__ void col_tile(const Tiles &T, int &b, int &i0, int &j
   const int tz = t / T.nty[b];
   i0 = tx * kTX;
   j0 = ty * kTY;
-  k0 = tz * kFluxKC;
+  k0 = tz * kc;
 }
 
 // Shared-memory plan of a column kernel (elements): x faces [NV][kTY][kTX+1]
@@ -310,17 +311,18 @@ __device__ __forceinline__ void col_faces64(const DevBlock &B, int i0, int j0, i
 }
 
 template <class C>
-__global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__restrict__ blks, Tiles T) {
+__global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__restrict__ blks, Tiles T,
+                                                               int kc) {
   constexpr int NV = C::nv;
   extern __shared__ double sm64[];
   int b, i0, j0, k0;
-  col_tile(T, b, i0, j0, k0);
+  col_tile(T, kc, b, i0, j0, k0);
   const DevBlock &B = blks[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = i0 + lane, j = j0 + warp;
   const bool cell = warp < kTY && i < B.mx && j < B.my;
   const int64_t szd = B.D.size;
-  const int k1 = min(k0 + kFluxKC, B.mz);
+  const int k1 = min(k0 + kc, B.mz);
   for (int k = k0; k < k1; ++k) {
     double dq[NV];
     int64_t n = 0, nd = 0;
@@ -335,6 +337,54 @@ __global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__
     OSTC_UNROLL for (int l = 0; l < NV; ++l) B.dq[l * szd + nd] = dq[l];
     local_time_step<C>(B, i, j, k, n, nd);
   }
+}
+
+// The same flux differences for grids too small to fill the GPU, where the
+// faces a thread evaluates one after another are what takes the time: a CTA
+// owns a row of 32 cells and each of its warps evaluates one face of every
+// cell (low and high in x, y and z, inviscid and viscous: 12 warps, 8 in 2-D)
+// into shared memory; the warps then add the differences, one variable each,
+// in the order of k_flux.  Twice the face evaluations of k_flux_col, one deep
+// instead of six per plane: 24 x 16 x 8 cells of the reacting layer take 24 us
+// instead of 652, the 48 x 24 ramp 12 us instead of 19.
+constexpr int kRowFaces = 6;
+
+template <class C>
+__global__ void __launch_bounds__(2 * kRowFaces * 32, C::mix == 0 ? 2 : 1)
+    k_flux_row(const DevBlock *__restrict__ blks, Tiles T) {
+  constexpr int NV = C::nv;
+  __shared__ double sm[2 * kRowFaces * NV * 32];
+  int b;
+  int t = tile_of(T, blockIdx.x, b);
+  const int tx = t % T.ntx[b];
+  t /= T.ntx[b];
+  const DevBlock &B = blks[b];
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const int i = tx * 32 + lane, j = t % T.nty[b], k = t / T.nty[b];
+  const int n_face = B.mz > 1 ? kRowFaces : kRowFaces - 2;
+  const bool cell = i < B.mx, visc = cP.viscous_order != 0;
+  const int64_t n = B.G.at(i, j, k), nd = B.D.at(i, j, k), szd = B.D.size;
+  if (cell && w < (visc ? 2 * n_face : n_face)) {
+    const int f = w < n_face ? w : w - n_face, d = f >> 1;
+    const int64_t s = d == 0 ? 1 : (d == 1 ? B.G.sx : B.G.sxy), nl = (f & 1) ? n : n - s;
+    double v[NV];
+    if (w < n_face)
+      inviscid_face<C>(B, nl, d, s, v);
+    else
+      viscous_face<C>(B, nl, d, s, v);
+    OSTC_UNROLL for (int l = 0; l < NV; ++l) sm[(w * NV + l) * 32 + lane] = v[l];
+  }
+  __syncthreads();
+  if (!cell) return;
+  for (int l = w; l < NV; l += blockDim.y) {
+    double dq = B.dq[l * szd + nd];
+    for (int f = 0; f < n_face; f += 2) dq -= sm[((f + 1) * NV + l) * 32 + lane] - sm[(f * NV + l) * 32 + lane];
+    if (visc)
+      for (int f = n_face; f < 2 * n_face; f += 2)
+        dq += sm[((f + 1) * NV + l) * 32 + lane] - sm[(f * NV + l) * 32 + lane];
+    B.dq[l * szd + nd] = dq;
+  }
+  if (w == blockDim.y - 1) local_time_step<C>(B, i, j, k, n, nd);
 }
 
 // ---------------------------------------------------------------- implicit

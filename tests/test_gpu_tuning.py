@@ -74,3 +74,26 @@ def test_fp64_flux_forms_agree_on_the_ramp(case_factory):
     assert err == ref_err
     for f in ref:
         assert np.array_equal(got[f][0], ref[f][0], equal_nan=True), f
+
+
+@pytest.mark.parametrize("precision,dims", [
+    ("fp64", (48, 24, 1)), ("fp64", (256, 128, 1)),  # rows, columns in 2-D
+    ("fp64", (33, 9, 7)), ("fp64", (96, 64, 32)),    # rows with remainders, short columns
+    ("mixed", (33, 9, 7)), ("mixed", (96, 64, 32)),  # marches of one cell, of a few
+])
+def test_grid_dependent_cuts_give_the_same_fluxes(case_factory, precision, dims):
+    """However the launch cuts a grid of this size (rows, columns of a few
+    planes, short marches), every cell's dq and time step are those of the other
+    variants, bit for bit."""
+    mx, my, mz = dims
+    if mz == 1:
+        case = case_factory(f"cut_ramp_{mx}", cases.ramp_case, mx=mx, my=my, total_step=2, output_screen=1)
+        fields = ("bv", "dq", "dt_local")
+    else:
+        case = case_factory(f"cut_{mx}", cases.mixing_layer_case, mx=mx, my=my, mz=mz, total_step=2, output_screen=1)
+        fields = ("bv", "sv", "dq", "dt_local")
+    ref, _ = run(case, precision, 0, 1, steps=2, fields=fields)
+    for variant in (0,) if precision == "fp64" else (0, 2, 3):
+        got, _ = run(case, precision, 0, variant, steps=2, fields=fields)
+        for f in fields:
+            assert np.array_equal(got[f][0], ref[f][0], equal_nan=True), (variant, f)
