@@ -38,6 +38,7 @@ struct DevParams {
   double low[kMaxSpec * 7], high[kMaxSpec * 7];
   double lj_inv[kMaxSpec], vis_coeff[kMaxSpec];
   double wq[kMaxSpec * kMaxSpec], w8[kMaxSpec * kMaxSpec];
+  int one;  // 1, where the compiler must not know an exponent
   int label[kMaxReac], order[kMaxReac];
   signed char sf[kMaxReac * kMaxSpec], sb[kMaxReac * kMaxSpec];
   double A[kMaxReac], b[kMaxReac], Ea[kMaxReac], A2[kMaxReac], b2[kMaxReac], Ea2[kMaxReac];

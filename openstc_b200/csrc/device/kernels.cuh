@@ -4,6 +4,10 @@
 // kernels take a Tiles work table so one launch covers every grid block.
 #pragma once
 
+#include <type_traits>
+#include <utility>
+
+#include "mechanism.hpp"
 #include "physics.cuh"
 
 namespace ostc {
@@ -144,8 +148,13 @@ __device__ __forceinline__ double sst_mut(const DevBlock &B, int64_t n, double m
 // A T^b exp(-Ea/T) evaluated as (A T^b) exp(-Ea/T), src/FiniteRateChem.cu:110-112.
 // pow(T, 0) and exp(-0/T) are exactly 1, so those calls are skipped without
 // changing a bit of the result.
+// One copy of pow in a kernel: the unrolled chemistry takes it 25 times, and
+// inlined the code no longer fits the instruction cache (5.5 of 12 stall cycles
+// per instruction were waits for instructions).
+static __device__ __noinline__ double pow_call(double x, double y) { return std::pow(x, y); }
+
 __device__ __forceinline__ double arrhenius_pow(double t, double A, double b) {
-  return b != 0 ? A * std::pow(t, b) : A;
+  return b != 0 ? A * pow_call(t, b) : A;
 }
 
 __device__ __forceinline__ double arrhenius(double t, double A, double b, double Ea) {
@@ -281,6 +290,204 @@ __device__ __forceinline__ void chemistry(double density, double t, const double
     omega_d[i] = od;
     omega[i] = creation - od;
   }
+}
+
+// Calls f(std::integral_constant<int, 0>), ..., f(<N - 1>).
+template <int N, class F>
+__device__ __forceinline__ void static_for(F &&f) {
+  [&]<int... Q>(std::integer_sequence<int, Q...>) {
+    (f(std::integral_constant<int, Q>{}), ...);
+  }(std::make_integer_sequence<int, N>{});
+}
+
+// chemistry<NS, FAST> for a mechanism whose stoichiometry M is known at
+// compile time: the same sums and products in the same order without their
+// zero terms and integer conversions, and (T-dependent only) the powers of
+// p_atm / RT of K_c once per reaction order.  Stored products are rounded
+// (__dmul_rn) as the general form's stores round them.
+template <class M, bool FAST>
+__device__ __forceinline__ void chemistry_fixed(double density, double t, const double *Y, double *omega,
+                                                double *omega_d, double *q1, double *q2, int st) {
+  constexpr int NS = M::ns;
+  const double ln_t = FAST ? std::log(t) : 0.0, t_inv = FAST ? 1.0 / t : 0.0;
+  auto rate1 = [&](int r) { return FAST ? arrhenius_exp(cP.A[r], cP.lnA[r], cP.b[r], cP.Ea[r], ln_t, t_inv)
+                                        : arrhenius(t, cP.A[r], cP.b[r], cP.Ea[r]); };
+  auto rate2 = [&](int r) { return FAST ? arrhenius_exp(cP.A2[r], cP.lnA2[r], cP.b2[r], cP.Ea2[r], ln_t, t_inv)
+                                        : arrhenius(t, cP.A2[r], cP.b2[r], cP.Ea2[r]); };
+  double c[NS];
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) c[l] = __dmul_rn(density * Y[l] / cP.mw[l], 1e-3);
+  double g[NS];
+  if constexpr (FAST)
+    gibbs_rt_fast<NS>(t, ln_t, t_inv, g);
+  else
+    gibbs_rt<NS>(t, g);
+  constexpr double temp_p = kDP_atm / kDR_u * 1e-3;
+  const double temp_t = temp_p / t;
+  const double ln_temp_t = FAST ? std::log(temp_p) - ln_t : 0.0;
+  // (p_atm / RT)^-1 and ^1 (other orders: as they come), and the powers of the
+  // concentrations once per species: pow(c, 1) is not always c bit for bit, and
+  // the general form takes the power of every exponent
+  double pt_m = 1.0, pt_p = 1.0, pow1[NS], pow2[NS];
+  if constexpr (!FAST) {
+    constexpr auto uses = [](int k, int e) {
+      for (int r = 0; r < M::nr; ++r)
+        if (M::sf[r][k] == e || M::sb[r][k] == e) return true;
+      return false;
+    };
+    static_for<NS>([&](auto kc) {
+      constexpr int k = kc;
+      if constexpr (uses(k, 1)) pow1[k] = pow_call(c[k], cP.one);
+      if constexpr (uses(k, 2)) pow2[k] = pow_call(c[k], 2 * cP.one);
+    });
+    static_for<M::nr>([&](auto rc) {
+      constexpr int r = rc;
+      constexpr auto first = [](int o) { int q = 0; while (q < M::nr && M::order(q) != o) ++q; return q; };
+      if constexpr (r == first(-1)) pt_m = pow_call(temp_t, cP.order[r]);
+      if constexpr (r == first(1)) pt_p = pow_call(temp_t, cP.order[r]);
+    });
+  }
+  static_for<M::nr>([&](auto rc) {
+    constexpr int r = rc, type = M::label[r], order = M::order(r);
+    double kf = rate1(r);
+    if constexpr (type == 3) {
+      if constexpr (FAST) {
+        kf += rate2(r);
+      } else {
+        const double e2 = cP.Ea2[r] != 0 ? std::exp(-cP.Ea2[r] / t) : 1.0;
+        kf = __fma_rn(arrhenius_pow(t, cP.A2[r], cP.b2[r]), e2, kf);
+      }
+    }
+    if constexpr (type > 3) {
+      double cc = 0;
+      OSTC_UNROLL for (int l = 0; l < NS; ++l) cc += c[l] * cP.tb[r * NS + l];
+      if constexpr (type == 4) {
+        kf *= cc;
+      } else {
+        const double kf_low = rate2(r);
+        const double kf_high = kf;
+        const double reduced_pressure = kf_low * cc / kf_high;
+        double F = 1.0;
+        if constexpr (type > 5) {
+          double f_cent = (1 - cP.troe_a[r]) * std::exp(-t / cP.troe_t3[r]) + cP.troe_a[r] * std::exp(-t / cP.troe_t1[r]);
+          if constexpr (type == 7) f_cent += std::exp(-cP.troe_t2[r] / t);
+          const double logFc = std::log10(f_cent);
+          const double cq = -0.4 - 0.67 * logFc;
+          const double nq = 0.75 - 1.27 * logFc;
+          const double logPr = std::log10(reduced_pressure);
+          const double tempo = (logPr + cq) / (nq - 0.14 * (logPr + cq));
+          const double pq = logFc / (1.0 + tempo * tempo);
+          F = FAST ? std::exp(pq * 2.302585092994045684) : pow_call(10, pq);
+        }
+        kf = kf_high * reduced_pressure / (1.0 + reduced_pressure) * F;
+      }
+    }
+    double kb;
+    if constexpr (type != 2) {
+      double d_gibbs = 0;
+      static_for<NS>([&](auto lc) {
+        constexpr int l = lc;
+        if constexpr (M::nu(r, l) != 0) d_gibbs += g[l] * M::nu(r, l);
+      });
+      if constexpr (FAST) {
+        kb = kf * std::exp(d_gibbs - order * ln_temp_t);
+      } else {
+        double kc = std::exp(-d_gibbs);
+        if constexpr (order == -1)
+          kc *= pt_m;
+        else if constexpr (order == 1)
+          kc *= pt_p;
+        else if constexpr (order != 0)
+          kc *= pow_call(temp_t, cP.order[r]);
+        kb = kf / kc;
+      }
+    } else {
+      kb = rate2(r);
+    }
+    double a1 = 1.0, a2 = 1.0;
+    static_for<NS>([&](auto jc) {
+      constexpr int j = jc, ef = M::sf[r][j], eb = M::sb[r][j];
+      static_assert(ef <= 2 && eb <= 2);
+      if constexpr (ef != 0) a1 *= FAST ? ipow(c[j], ef) : (ef == 1 ? pow1[j] : pow2[j]);
+      if constexpr (eb != 0) a2 *= FAST ? ipow(c[j], eb) : (eb == 1 ? pow1[j] : pow2[j]);
+    });
+    q1[r * st] = __dmul_rn(a1, kf);
+    q2[r * st] = __dmul_rn(a2, kb);
+  });
+  static_for<NS>([&](auto ic) {
+    constexpr int i = ic;
+    double creation = 0, od = 0;
+    static_for<M::nr>([&](auto rc) {
+      constexpr int r = rc, f = M::sf[r][i], bb = M::sb[r][i];
+      if constexpr (f != 0 && bb != 0) {
+        creation += q2[r * st] * f + q1[r * st] * bb;
+        od += q1[r * st] * f + q2[r * st] * bb;
+      } else if constexpr (f != 0) {
+        creation += q2[r * st] * f;
+        od += q1[r * st] * f;
+      } else if constexpr (bb != 0) {
+        creation += q1[r * st] * bb;
+        od += q2[r * st] * bb;
+      }
+    });
+    const double w = cP.mw[i] * 1e+3;
+    od = __dmul_rn(od, w);
+    omega[i] = __fma_rn(creation, w, -od);  // as the general form contracts
+    omega_d[i] = od;
+  });
+}
+
+// Row m of the same sum for a run-time mechanism: only the reactions that
+// change species m are visited.
+template <int NS>
+__device__ __forceinline__ void jacobian_row(int m, const double *q1, const double *q2, int st, double *zz) {
+  OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] = 0;
+  for (int r = 0; r < cP.nr; ++r) {
+    const int dn = cP.sb[r * NS + m] - cP.sf[r * NS + m];
+    if (dn == 0) continue;
+    const double a1 = q1[r * st], a2 = q2[r * st];
+    OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] += dn * (cP.sf[r * NS + q] * a1 - cP.sb[r * NS + q] * a2);
+  }
+}
+
+// M: a compile-time mechanism, or void for the case's own tables.
+template <int NS, bool FAST, class M>
+__device__ __forceinline__ void chemistry_of(double density, double t, const double *Y, double *omega, double *omega_d,
+                                             double *q1, double *q2, int st) {
+  if constexpr (std::is_void_v<M>)
+    chemistry<NS, FAST>(density, t, Y, omega, omega_d, q1, q2, st);
+  else
+    chemistry_fixed<M, FAST>(density, t, Y, omega, omega_d, q1, q2, st);
+}
+
+// Row m of sum_r nu_mr (sf_qr q1_r - sb_qr q2_r), the EPI Jacobian before its
+// scaling, over the reactions of M that change species m and the species
+// they involve; each entry sums its terms in reaction order.
+template <class M, int m>
+__device__ __forceinline__ void jacobian_row_fixed(const double *q1, const double *q2, int st, double *zz) {
+  static_for<M::ns>([&](auto qc) { zz[qc] = 0; });
+  static_for<M::nr>([&](auto rc) {
+    constexpr int r = rc, dn = M::nu(r, m);
+    if constexpr (dn != 0) {
+      const double a1 = q1[r * st], a2 = q2[r * st];
+      static_for<M::ns>([&](auto qc) {
+        constexpr int q = qc, f = M::sf[r][q], b = M::sb[r][q];
+        if constexpr (f != 0 && b != 0)
+          zz[q] += dn * (f * a1 - b * a2);
+        else if constexpr (f != 0)
+          zz[q] += (dn * f) * a1;
+        else if constexpr (b != 0)
+          zz[q] -= (dn * b) * a2;
+      });
+    }
+  });
+}
+
+template <int NS, class M, int m>
+__device__ __forceinline__ void jacobian_row_of(const double *q1, const double *q2, int st, double *zz) {
+  if constexpr (std::is_void_v<M>)
+    jacobian_row<NS>(m, q1, q2, st, zz);
+  else
+    jacobian_row_fixed<M, m>(q1, q2, st, zz);
 }
 
 // ---------------------------------------------------------------- inviscid

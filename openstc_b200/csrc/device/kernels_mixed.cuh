@@ -497,7 +497,7 @@ __device__ __forceinline__ void sst_source(const DevBlock &B, int64_t n, double 
 // Arrhenius rate as one exponential):
 // returns dq species = J omega and writes the EPI / DA Jacobian.  q1, q2:
 // this thread's column of the CTA's shared rate arrays (stride kCta).
-template <class C>
+template <class C, class M>
 __device__ __forceinline__ void chem_cell(const DevBlock &B, int64_t n, int64_t nz, double *q1, double *q2,
                                           double *dq_spec) {
   constexpr int NS = C::ns;
@@ -505,36 +505,29 @@ __device__ __forceinline__ void chem_cell(const DevBlock &B, int64_t n, int64_t 
   double Y[NS], omega[NS], omega_d[NS];
   OSTC_UNROLL for (int l = 0; l < NS; ++l) Y[l] = ld(B.sv + l * sz + n);
   const double density = ld(B.bv + n), t = ld(B.bv + 5 * sz + n);
-  chemistry<NS, true>(density, t, Y, omega, omega_d, q1, q2, kCta);
+  chemistry_of<NS, true, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
   const double jac = ld(B.jac + n);
   OSTC_UNROLL for (int l = 0; l < NS; ++l) dq_spec[l] = jac * omega[l];
   const int method = cP.chem_src_method;
   if (method == 1) {
-    // compute_chem_src_jacobian with the reaction loop outside the species
-    // loop: each row m visits only the reactions that change species m once,
-    // and every (m, q) entry still sums its terms in reaction order
-    const int nr = cP.nr, na = cP.na;
+    // compute_chem_src_jacobian, row by row
+    const int na = cP.na;
     // 1 / (rho Y_q) once per species (0 below the floor): products, not
     // NS^2 divisions, within an ulp of the FP64 path's quotients
     double inv_rho_y[NS];
     OSTC_UNROLL for (int q = 0; q < NS; ++q) inv_rho_y[q] = Y[q] > 1e-25 ? 1.0 / (density * Y[q]) : 0.0;
     // only the leading na x na block (the other rows and columns are zero)
-    OSTC_UNROLL for (int m = 0; m < NS; ++m) {
-      if (m >= na) break;
+    static_for<NS>([&](auto mc) {
+      constexpr int m = mc;
+      if (m >= na) return;
       double zz[NS];
-      OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] = 0;
-      for (int r = 0; r < nr; ++r) {
-        const int dn = cP.sb[r * NS + m] - cP.sf[r * NS + m];
-        if (dn == 0) continue;
-        const double a1 = q1[r * kCta], a2 = q2[r * kCta];
-        OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] += dn * (cP.sf[r * NS + q] * a1 - cP.sb[r * NS + q] * a2);
-      }
+      jacobian_row_of<NS, M, m>(q1, q2, kCta, zz);
       OSTC_UNROLL for (int q = 0; q < NS; ++q) {
         if (q >= na) break;
         const double v = zz[q] * inv_rho_y[q];
         B.chem_jac[(m * na + q) * sz0 + nz] = cP.mw[m] * v * 1e+3;
       }
-    }
+    });
   } else if (method == 2) {
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
       double v = 0;
@@ -549,7 +542,7 @@ __device__ __forceinline__ void chem_cell(const DevBlock &B, int64_t n, int64_t 
 // (chem_quiet set) the chemistry of the cells it did not judge quiet runs in
 // k_chem_list over a compacted list instead, with every lane of a warp busy;
 // here those cells get zero species source, which k_chem_list overwrites.
-template <class C>
+template <class C, class M>
 __global__ void __launch_bounds__(kCta, 4) k_source_mx(const DevBlock *__restrict__ blks, Tiles T) {
   constexpr int NS = C::ns, NV = C::nv;
   extern __shared__ double sq[];
@@ -583,7 +576,7 @@ __global__ void __launch_bounds__(kCta, 4) k_source_mx(const DevBlock *__restric
       }
     } else {
       const int tid = threadIdx.x + kTX * (threadIdx.y + kTY * threadIdx.z);
-      chem_cell<C>(B, n, nz, sq + tid, sq + cP.nr * kCta + tid, dq + 5);
+      chem_cell<C, M>(B, n, nz, sq + tid, sq + cP.nr * kCta + tid, dq + 5);
     }
   }
   OSTC_UNROLL for (int l = 0; l < NV; ++l) B.dq[l * szd + nd] = dq[l];
@@ -615,7 +608,7 @@ __global__ void __launch_bounds__(256) k_chem_compact(const DevBlock *__restrict
 
 // Chemistry of the listed cells (k_chem_compact), one thread per entry, full
 // warps; launched for the block's cell count, entries past the list return.
-template <class C>
+template <class C, class M>
 __global__ void __launch_bounds__(kCta, 4) k_chem_list(const DevBlock *__restrict__ blks, int b,
                                                        const int *__restrict__ list, const int *count) {
   constexpr int NS = C::ns;
@@ -628,7 +621,7 @@ __global__ void __launch_bounds__(kCta, 4) k_chem_list(const DevBlock *__restric
             k = static_cast<int>(c / (static_cast<int64_t>(B.mx) * B.my));
   const int64_t n = B.G.at(i, j, k), nz = B.Z.at(i, j, k), nd = B.D.at(i, j, k), szd = B.D.size;
   double dqs[NS];
-  chem_cell<C>(B, n, nz, sq + threadIdx.x, sq + cP.nr * kCta + threadIdx.x, dqs);
+  chem_cell<C, M>(B, n, nz, sq + threadIdx.x, sq + cP.nr * kCta + threadIdx.x, dqs);
   OSTC_UNROLL for (int l = 0; l < NS; ++l) B.dq[(5 + l) * szd + nd] = dqs[l];
 }
 

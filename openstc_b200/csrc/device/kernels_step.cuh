@@ -11,7 +11,7 @@ constexpr int kCta = kTX * kTY * kTZ;
 // ---------------------------------------------------------------- source
 // compute_source (src/SourceTerm.cuh:11-40) fused with the reset of dq:
 // writes every dq component of an interior cell (zero + source).
-template <class C>
+template <class C, class M>
 __global__ void __launch_bounds__(kCta, 4) k_source(const DevBlock *__restrict__ blks, Tiles T) {
   constexpr int NS = C::ns, NV = C::nv;
   extern __shared__ double sq[];  // q1, q2: 2 * n_reac * kCta doubles
@@ -52,31 +52,24 @@ __global__ void __launch_bounds__(kCta, 4) k_source(const DevBlock *__restrict__
     double Y[NS], omega[NS], omega_d[NS];
     OSTC_UNROLL for (int l = 0; l < NS; ++l) Y[l] = ld(B.sv + l * sz + n);
     const double density = ld(B.bv + n), t = ld(B.bv + 5 * sz + n);
-    chemistry<NS>(density, t, Y, omega, omega_d, q1, q2, kCta);
+    chemistry_of<NS, false, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
     const double jac = ld(B.jac + n);
     OSTC_UNROLL for (int l = 0; l < NS; ++l) dq[l + 5] = 0.0 + jac * omega[l];
     const int method = cP.chem_src_method;
     if (method == 1) {
       // compute_chem_src_jacobian, src/FiniteRateChem.cu:173-194
-      // the reaction loop sits outside the species loop: each row m visits
-      // only the reactions that change species m (the others add an exact
-      // zero in the reference), and every (m, q) entry still sums its terms
-      // in reaction order, so the entries are the reference's bit for bit
-      const int nr = cP.nr;
-      OSTC_UNROLL for (int m = 0; m < NS; ++m) {
+      // each row visits only the reactions that change its species (the
+      // others add an exact zero in the reference) and sums its terms in
+      // reaction order, so the entries are the reference's bit for bit
+      static_for<NS>([&](auto mc) {
+        constexpr int m = mc;
         double zz[NS];
-        OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] = 0;
-        for (int r = 0; r < nr; ++r) {
-          const int dn = cP.sb[r * NS + m] - cP.sf[r * NS + m];
-          if (dn == 0) continue;
-          const double a1 = q1[r * kCta], a2 = q2[r * kCta];
-          OSTC_UNROLL for (int q = 0; q < NS; ++q) zz[q] += dn * (cP.sf[r * NS + q] * a1 - cP.sb[r * NS + q] * a2);
-        }
+        jacobian_row_of<NS, M, m>(q1, q2, kCta, zz);
         OSTC_UNROLL for (int q = 0; q < NS; ++q) {
           const double v = Y[q] > 1e-25 ? zz[q] / (density * Y[q]) : 0.0;
           B.chem_jac[(m * NS + q) * sz0 + nz] = cP.mw[m] * v * 1e+3;
         }
-      }
+      });
     } else if (method == 2) {
       OSTC_UNROLL for (int l = 0; l < NS; ++l) {
         double v = 0;

@@ -74,30 +74,22 @@ inline JudgeTables make_judge_tables(const DevParams &p) {
 // One FP64 EPI step at fixed density: rho dY = (I - dt J)^-1 dt omega, with
 // omega and J as the solver computes them (finite_rate_chemistry and
 // compute_chem_src_jacobian, src/FiniteRateChem.cu:7-194; EPI, :211-234).
-template <int NS>
+template <int NS, class M = void>
 __device__ inline void epi_increment(double T, double rho, const double *Y, double dt, double *q1, double *q2,
                                      int stride, double *dy) {
   double omega[NS], omega_d[NS];
-  chemistry<NS>(rho, T, Y, omega, omega_d, q1, q2, stride);
+  chemistry_of<NS, false, M>(rho, T, Y, omega, omega_d, q1, q2, stride);
   double lhs[NS * NS];
-  const int nr = cP.nr;
-  for (int m = 0; m < NS; ++m) {
-    // reactions outside the species loop (each (m, q) still sums in reaction
-    // order), as in k_source
+  static_for<NS>([&](auto mc) {
+    constexpr int m = mc;
     double zz[NS];
-    for (int q = 0; q < NS; ++q) zz[q] = 0;
-    for (int r = 0; r < nr; ++r) {
-      const int dn = cP.sb[r * NS + m] - cP.sf[r * NS + m];
-      if (dn == 0) continue;
-      const double a1 = q1[r * stride], a2 = q2[r * stride];
-      for (int q = 0; q < NS; ++q) zz[q] += dn * (cP.sf[r * NS + q] * a1 - cP.sb[r * NS + q] * a2);
-    }
-    for (int q = 0; q < NS; ++q) {
+    jacobian_row_of<NS, M, m>(q1, q2, stride, zz);
+    OSTC_UNROLL for (int q = 0; q < NS; ++q) {
       const double v = Y[q] > 1e-25 ? zz[q] / (rho * Y[q]) : 0.0;
       const double J = cP.mw[m] * v * 1e+3;
       lhs[m * NS + q] = (m == q ? 1.0 : 0.0) - dt * J;
     }
-  }
+  });
   int piv[NS];
   lu_factor<NS>(lhs, piv);
   double x[NS];

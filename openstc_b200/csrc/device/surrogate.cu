@@ -142,6 +142,7 @@ __global__ void k_sample(double *states, int64_t n, uint64_t seed, DevBlock F, i
   o[11] = dt;
 }
 
+template <class M>
 __global__ void __launch_bounds__(128) k_label(const double *states, double *dy, int64_t n) {
   extern __shared__ double sq[];
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(128) k_label(const double *states, double *dy,
     mw_inv += Y[k] / cP.mw[k];
   }
   const double rho = s[1] / (kDR_u * s[0] * mw_inv);
-  sur::epi_increment<NS>(s[0], rho, Y, s[11], sq + threadIdx.x, sq + cP.nr * blockDim.x + threadIdx.x, blockDim.x, d);
+  sur::epi_increment<NS, M>(s[0], rho, Y, s[11], sq + threadIdx.x, sq + cP.nr * blockDim.x + threadIdx.x, blockDim.x, d);
   for (int k = 0; k < NS; ++k) dy[i * NS + k] = d[k];
 }
 
@@ -325,7 +326,13 @@ void Surrogate::pack() {
   packed_ = true;
 }
 
-static size_t label_smem(const DevParams &p) { return 2 * static_cast<size_t>(p.nr) * 128 * sizeof(double); }
+void Surrogate::launch_label(const double *states, double *dy, int64_t n) {
+  const size_t smem = 2 * static_cast<size_t>(chem_.nr) * 128 * sizeof(double);  // two rates per reaction and thread
+  auto *fn = mech::matches<mech::H2O2>(chem_) ? k_label<mech::H2O2> : k_label<void>;
+  ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "smem");
+  fn<<<(n + 127) / 128, 128, smem, stream_>>>(states, dy, n);
+  ck(cudaGetLastError(), "label launch");
+}
 
 void Surrogate::generate(int64_t n, uint64_t seed, const DevBlock *field, double field_fraction) {
   if (n <= 0) throw std::runtime_error("number of samples must be positive");
@@ -348,10 +355,7 @@ void Surrogate::generate(int64_t n, uint64_t seed, const DevBlock *field, double
   if (field) F = *field;
   k_sample<<<(n + 255) / 256, 256, 0, stream_>>>(states_, n, seed, F, field ? 1 : 0, field_fraction, gate);
   ck(cudaGetLastError(), "sample launch");
-  const size_t smem = label_smem(chem_);
-  ck(cudaFuncSetAttribute(k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "smem");
-  k_label<<<(n + 127) / 128, 128, smem, stream_>>>(states_, labels_, n);
-  ck(cudaGetLastError(), "label launch");
+  launch_label(states_, labels_, n);
   // normalisation from the data
   DevTemp<double> acc(2 * kSurIn + kSurOut, "cudaMalloc stats");
   ck(cudaMemsetAsync(acc.p, 0, (2 * kSurIn + kSurOut) * sizeof(double), stream_), "memset stats");
@@ -619,10 +623,7 @@ void Surrogate::label_host(const double *states, int64_t n, double *dy) {
   DevTemp<double> s_buf(n * kSurIn, "label alloc"), d_buf(n * NS, "label alloc");
   double *s = s_buf.p, *d = d_buf.p;
   ck(cudaMemcpyAsync(s, states, n * kSurIn * 8, cudaMemcpyHostToDevice, stream_), "label upload");
-  const size_t smem = label_smem(chem_);
-  ck(cudaFuncSetAttribute(k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "smem");
-  k_label<<<(n + 127) / 128, 128, smem, stream_>>>(s, d, n);
-  ck(cudaGetLastError(), "label");
+  launch_label(s, d, n);
   ck(cudaMemcpyAsync(dy, d, n * NS * 8, cudaMemcpyDeviceToHost, stream_), "label download");
   ck(cudaStreamSynchronize(stream_), "label");
 }

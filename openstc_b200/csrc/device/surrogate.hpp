@@ -117,6 +117,7 @@ class Surrogate {
   void reduce(float *grad, double lr, double *loss);
   void pack();
   void upload_chem();
+  void launch_label(const double *states, double *dy, int64_t n);
   void features(const double *states_dev, int64_t n, uint16_t *x_dev, float *t_dev, const double *dy_dev);
   DevParams chem_;
   std::vector<int> elem_comp_;

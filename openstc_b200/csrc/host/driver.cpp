@@ -247,6 +247,7 @@ void Driver::build_dev_params() {
   const Parameter &P = parameter;
   p.ns = spec.n_spec;
   p.nr = reac.n_reac;
+  p.one = 1;
   if (p.nr > kMaxReac) throw ParameterError("at most 50 reactions are supported (MAX_REAC_NUMBER)");
   p.n_var = P.get_int("n_var");
   p.n_scalar = P.get_int("n_scalar");

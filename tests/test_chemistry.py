@@ -129,3 +129,21 @@ def test_epi_increment_conserves_mass(params):
                                    dY.ctypes.data_as(C.POINTER(C.c_double)))
     assert np.max(np.abs(dY[:9])) > 0
     assert abs(dY[:9].sum()) < 1e-12 * np.max(np.abs(dY[:9]))
+
+
+def test_compile_time_mechanism_is_the_shipped_one(params):
+    """The stoichiometry the chemistry kernels unroll over (mechanism.hpp) is
+    that of the mechanism file, or the shipped cases would take the general
+    loops."""
+    import re
+    from pathlib import Path
+
+    text = (Path(ostc.__file__).parent / "csrc" / "device" / "mechanism.hpp").read_text()
+
+    def table(name):
+        body = text[text.index(name):].split("=", 1)[1].split(";", 1)[0]
+        return [int(v) for v in re.findall(r"-?\d+", body)]
+
+    assert table("label[nr]") == list(params.label[:19])
+    assert table("sf[nr][ns]") == list(params.stoi_f[:19 * 9])
+    assert table("sb[nr][ns]") == list(params.stoi_b[:19 * 9])
