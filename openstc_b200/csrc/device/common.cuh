@@ -8,6 +8,8 @@
 
 #include <cstdint>
 
+#include <vector_types.h>
+
 #ifdef __CUDACC__
 #define OSTC_HD __host__ __device__
 #else
@@ -76,25 +78,28 @@ struct DevBlock {
   double *chem_jac, *turb_src_jac;
   unsigned char *lu_piv;
   double *dq, *dq0, *dqk, *inv_spec, *visc_spec, *dt_local, *bv_last;
-  // species enthalpies h_k(T) of each cell, written by k_dq0 for the DPLUR
-  // sweeps (layout D, ns components; mixtures under DPLUR only)
-  double *h_spec;
-  // FP32-bulk path under DPLUR: the species enthalpies (k_dq0, instead of
-  // h_spec) and the inviscid spectral radii (the x flux pass, beside
-  // inv_spec) in FP32, the precision the sweeps use them in; layout D
-  float *h_spec32, *inv_spec32;
+  // DPLUR, layout D (FP64 path): the species enthalpies h_k(T) of each cell
+  // (k_dq0) and the terms of its flux-Jacobian product that no direction
+  // enters (sweep_terms): [0] the total enthalpy, [1 + 2 s], [2 + 2 s] the
+  // pressure terms of the increments in buffer s (0 dq, 1 dq0, 2 dqk)
+  double *h_spec, *terms;
+  // the same on the FP32-bulk path: the weights of the species increments in
+  // the pressure term (ns components, k_dq0), the pressure term of dqf[s]
+  // ([s]), and the inviscid spectral radii with the total enthalpy (k_dq0)
+  float *weight32, *terms32;
+  float4 *radii32;
   // chemistry surrogate (layout Z; null when off): cells the surrogate judged
   // chemically quiet take its increment rate rho dY/dt as an explicit source
   unsigned char *chem_quiet;
   double *chem_rate;
-  // FP32-bulk path under DPLUR: the increments in FP32 (layout D, nv
-  // components each): [0] dq0, [1] and [2] the ping-pong of the sweeps; the
-  // last sweep writes the FP64 dq.  Null on the FP64 path.
-  float *dqf[3];
+  // FP32-bulk path under DPLUR: the increments in FP32 (layout D, four quads
+  // each, store_increments32): [0] dq0, [1] and [2] the ping-pong of the
+  // sweeps; the last sweep writes the FP64 dq.  Null on the FP64 path.
+  float4 *dqf[3];
   // FP32-bulk path: an FP32 copy (layout G) of every operand of the
-  // direction-pass flux kernels, component by component (fp32::F32); null on
-  // the FP64 path
-  float *f32;
+  // direction-pass flux kernels, four components together (fp32::Quad); null
+  // on the FP64 path
+  float4 *f32;
   // with exact inner faces: bit 2 d + (1 for the high side) is set when that
   // block face is an inner face whose neighbours the DPLUR sweeps take
   int inner_mask;

@@ -86,7 +86,12 @@ class EngineT final : public Engine {
     source_smem_ = C::mix == 2 ? 2 * std::max(1, s.params.nr) * kCta * sizeof(double) : 0;
     flux_smem_ = C::nv * kCta * (C::mixed ? sizeof(float) : sizeof(double));
     col_smem_ = sizeof(double) * ColSmem<C::nv>::size;
-    dq0_smem_ = (C::mix == 2 && s.params.chem_src_method == 1) ? sizeof(double) * C::ns * C::ns * kCta : 0;
+    // the EPI matrix, a slice per thread
+    dq0_smem_ = 0;
+    if (C::mix == 2 && s.params.chem_src_method == 1) {
+      const int n = C::mixed && s.params.na == C::ns - 1 ? C::ns - 1 : C::ns;
+      dq0_smem_ = sizeof(double) * n * n * kCta;
+    }
     if (dq0_smem_ > 48 * 1024)
       cuda_check(cudaFuncSetAttribute(k_dq0<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(dq0_smem_)),
@@ -409,7 +414,7 @@ class EngineT final : public Engine {
     int n = 2;  // source, flux
     if constexpr (C::mixed) n += (p.dim == 3 ? 2 : 1) + static_cast<int>(blocks_.size());  // pack + one pass per direction
     if (p.implicit_method == 1) {
-      n += 1 + p.dplur_inner_step;
+      n += 1 + (p.dplur_inner_step > 0 ? 1 : 0) + p.dplur_inner_step;
     } else if ((C::mix == 2 && p.chem_src_method != 0) || (C::turb && p.turb_implicit == 1)) {
       n += 1;
     }
@@ -533,47 +538,41 @@ class EngineT final : public Engine {
       allocations_.push_back(q);
       ptr = static_cast<double *>(q);
     }
-    B.h_spec = nullptr;
-    B.h_spec32 = B.inv_spec32 = nullptr;
-    if (C::mix != 0 && p.implicit_method == 1 && !C::mixed) {
-      void *q = nullptr;
-      const size_t bytes = sizeof(double) * static_cast<size_t>(B.D.size) * C::ns;
-      cuda_check(cudaMalloc(&q, bytes), "cudaMalloc h_spec");
-      cuda_check(cudaMemset(q, 0, bytes), "memset h_spec");
-      allocations_.push_back(q);
-      B.h_spec = static_cast<double *>(q);
-    }
-    if (C::mixed && p.implicit_method == 1) {
-      auto falloc = [&](int n) {
+    B.h_spec = B.terms = nullptr;
+    B.weight32 = B.terms32 = nullptr;
+    B.radii32 = nullptr;
+    if (p.implicit_method == 1) {
+      auto alloc = [&](size_t bytes) {
         void *q = nullptr;
-        const size_t bytes = sizeof(float) * static_cast<size_t>(B.D.size) * n;
-        cuda_check(cudaMalloc(&q, bytes), "cudaMalloc fp32 spectra");
-        cuda_check(cudaMemset(q, 0, bytes), "memset fp32 spectra");
+        cuda_check(cudaMalloc(&q, bytes), "cudaMalloc sweep terms");
+        cuda_check(cudaMemset(q, 0, bytes), "memset sweep terms");
         allocations_.push_back(q);
-        return static_cast<float *>(q);
+        return q;
       };
-      if (C::mix != 0) B.h_spec32 = falloc(C::ns);
-      B.inv_spec32 = falloc(3);
-    }
-    for (auto &f : B.dqf) f = nullptr;
-    if (C::mixed && p.implicit_method == 1) {
-      for (auto &f : B.dqf) {
-        void *q = nullptr;
-        const size_t bytes = sizeof(float) * static_cast<size_t>(B.D.size) * C::nv;
-        cuda_check(cudaMalloc(&q, bytes), "cudaMalloc dqf");
-        cuda_check(cudaMemset(q, 0, bytes), "memset dqf");
-        allocations_.push_back(q);
-        f = static_cast<float *>(q);
+      const size_t n = static_cast<size_t>(B.D.size);
+      if constexpr (C::mixed) {
+        B.weight32 = static_cast<float *>(alloc(sizeof(float) * n * C::ns));
+        B.terms32 = static_cast<float *>(alloc(sizeof(float) * n * 3));
+        B.radii32 = static_cast<float4 *>(alloc(sizeof(float4) * n));
+      } else {
+        if (C::mix != 0) B.h_spec = static_cast<double *>(alloc(sizeof(double) * n * C::ns));
+        B.terms = static_cast<double *>(alloc(sizeof(double) * n * 7));
       }
     }
+    for (auto &f : B.dqf) f = nullptr;
     B.f32 = nullptr;
     if constexpr (C::mixed) {
-      void *q = nullptr;
-      const size_t bytes = sizeof(float) * static_cast<size_t>(B.G.size) * fp32::F32<C>::count;
-      cuda_check(cudaMalloc(&q, bytes), "cudaMalloc f32");
-      cuda_check(cudaMemset(q, 0, bytes), "memset f32");
-      allocations_.push_back(q);
-      B.f32 = static_cast<float *>(q);
+      auto quads = [&](const Lay &L, int n) {
+        void *q = nullptr;
+        const size_t bytes = sizeof(float4) * static_cast<size_t>(L.size) * n;
+        cuda_check(cudaMalloc(&q, bytes), "cudaMalloc quads");
+        cuda_check(cudaMemset(q, 0, bytes), "memset quads");
+        allocations_.push_back(q);
+        return static_cast<float4 *>(q);
+      };
+      if (p.implicit_method == 1)
+        for (auto &f : B.dqf) f = quads(B.D, C::nv / 4);
+      B.f32 = quads(B.G, fp32::Quad::count);
     }
     B.lu_piv = nullptr;
     if (C::mix == 2 && p.chem_src_method == 1) {
@@ -851,6 +850,10 @@ class EngineT final : public Engine {
     if (p.implicit_method == 1) {
       k_dq0<C><<<grid(tiles0_), block3(), dq0_smem_, stream_>>>(d_blocks_, tiles0_);
       mark("dq0");
+      if (p.dplur_inner_step > 0) {
+        k_sweep_terms<C><<<grid(tiles0_), block3(), 0, stream_>>>(d_blocks_, tiles0_);
+        mark("sweep_terms");
+      }
       if constexpr (C::mixed) {
         // FP32 increments dqf[0] (dq0) -> dqf[1] -> dqf[2] -> ..., the last
         // sweep into the FP64 dq (k_dq0 writes the FP64 dq0 when there is no sweep)
@@ -864,11 +867,11 @@ class EngineT final : public Engine {
         final_dq_ = p.dplur_inner_step > 0 ? 0 : 1;
       } else {
         int in = 1;
-        launch_halo(kHaloHspec);
+        launch_halo(kHaloEnthalpy);
         for (int s = 0; s < p.dplur_inner_step; ++s) {
           const int out = (s % 2 == 0) ? 2 : 0;
           launch_halo(kHaloDq, in);
-          k_sweep<C><<<grid(tiles0_), block3(), 0, stream_>>>(d_blocks_, tiles0_, in, out);
+          k_sweep<C><<<grid(tiles0_), block3(), 0, stream_>>>(d_blocks_, tiles0_, in, out, s + 1 == p.dplur_inner_step);
           mark("dplur_sweep");
           in = out;
         }

@@ -96,54 +96,21 @@ __device__ __forceinline__ void thermo(float t, float *h, float *cp) {
   }
 }
 
-// Where the FP32 kernels read their operands (index n of layout G):
-// Src64 converts the FP64 state arrays on load; Src32 reads their FP32 copy
-// (DevBlock::f32, written once per step by k_pack32 and, for the geometry,
-// once per run by k_pack32_static), half the bytes and no conversion.
-// prim(v, n): primitive v, 0..5 the basic variables (rho, u, v, w, p, T),
-// 6.. the scalars (Y_k, k, omega).
-struct Src64 {
-  const DevBlock &B;
-  __device__ __forceinline__ float prim(int v, int64_t n) const {
-    return ldf((v < 6 ? B.bv + v * B.G.size : B.sv + (v - 6) * B.G.size) + n);
-  }
-  __device__ __forceinline__ float metric(int q, int64_t n) const { return ldf(B.metric + q * B.G.size + n); }
-  __device__ __forceinline__ float jac(int64_t n) const { return ldf(B.jac + n); }
-  __device__ __forceinline__ float mul(int64_t n) const { return ldf(B.mul + n); }
-  __device__ __forceinline__ float mut(int64_t n) const { return ldf(B.mut + n); }
-  __device__ __forceinline__ float cond(int64_t n) const { return ldf(B.cond + n); }
-  __device__ __forceinline__ float tcond(int64_t n) const { return ldf(B.turb_cond + n); }
-  __device__ __forceinline__ float rho_d(int l, int64_t n) const { return ldf(B.rho_d + l * B.G.size + n); }
-  __device__ __forceinline__ float wall(int64_t n) const { return ldf(B.wall_dist + n); }
-  __device__ __forceinline__ float acoustic(int64_t n) const { return ldf(B.acoustic + n); }
-  __device__ __forceinline__ float gamma(int64_t n) const { return ldf(B.gamma + n); }
-};
-
-// Component offsets of the FP32 copy (each component B.G.size floats).
-template <class C>
-struct F32 {
-  static constexpr int prim = 0, mul = 6 + C::nsc, mut = mul + 1, cond = mul + 2, tcond = mul + 3, rho_d = mul + 4,
-                       acoustic = rho_d + C::ns, gamma = acoustic + 1,
-                       n_dynamic = gamma + 1,  // written every step
-                       wall = n_dynamic, jac = wall + 1, metric = jac + 1, count = metric + 9;
-};
-
-template <class C>
-struct Src32 {
-  const float *f;
-  int64_t sz;
-  __device__ __forceinline__ float at(int c, int64_t n) const { return __ldg(f + c * sz + n); }
-  __device__ __forceinline__ float prim(int v, int64_t n) const { return at(F32<C>::prim + v, n); }
-  __device__ __forceinline__ float metric(int q, int64_t n) const { return at(F32<C>::metric + q, n); }
-  __device__ __forceinline__ float jac(int64_t n) const { return at(F32<C>::jac, n); }
-  __device__ __forceinline__ float mul(int64_t n) const { return at(F32<C>::mul, n); }
-  __device__ __forceinline__ float mut(int64_t n) const { return at(F32<C>::mut, n); }
-  __device__ __forceinline__ float cond(int64_t n) const { return at(F32<C>::cond, n); }
-  __device__ __forceinline__ float tcond(int64_t n) const { return at(F32<C>::tcond, n); }
-  __device__ __forceinline__ float rho_d(int l, int64_t n) const { return at(F32<C>::rho_d + l, n); }
-  __device__ __forceinline__ float wall(int64_t n) const { return at(F32<C>::wall, n); }
-  __device__ __forceinline__ float acoustic(int64_t n) const { return at(F32<C>::acoustic, n); }
-  __device__ __forceinline__ float gamma(int64_t n) const { return at(F32<C>::gamma, n); }
+// The FP32 copy of the operands of the flux passes and the sweeps
+// (DevBlock::f32), written once per step by k_pack32 and, for the geometry,
+// once per run by k_pack32_static.  Four components of a cell lie together
+// (quads, one array of B.G.size float4 per quad), so that a stencil point is
+// a few 16-byte loads: a face reads 74 of them instead of 348 4-byte ones, and
+// those loads, with their address arithmetic, are what the passes waited for.
+struct Quad {
+  static constexpr int rho_vel = 0,    // rho, u, v, w
+      p_t_turb = 1,                    // p, T, k, omega
+      y0 = 2, y4 = 3,                  // Y_0..3, Y_4..7
+      y8_mu = 4,                       // Y_8, mu, mu_t, lambda
+      misc = 5,                        // lambda_t, a, gamma, (rho D)_8
+      d0 = 6, d4 = 7,                  // (rho D)_0..3, _4..7
+      n_dynamic = 8, metric = 8,       // metric + d: grad of coordinate d, and J, wall distance, 0
+      count = 11;
 };
 
 // h_k and cp_k of species i at t (thermo<> for one species)
@@ -162,77 +129,83 @@ __device__ __forceinline__ void thermo_one(int i, float t, float &h, float &cp) 
 }
 
 // ------------------------------------------------------------ inviscid face
-// The face functions read the primitive stencil through a reader, so that one
-// copy of the physics serves the kernels that load it from the FP64 arrays
-// and the one that stages it in shared memory.  Primitive index v: 0..5 the
-// basic variables (rho, u, v, w, p, T), 6.. the scalars (Y_k, k, omega);
-// flux variable l is primitive l below 5 and l + 1 from 5 on.
+// Left and right values at a face of a variable with these four stencil values.
+__device__ __forceinline__ void reconstruct(int rec, float pm, float p0, float p1, float p2, float &l, float &r) {
+  if (rec == 2 || rec == 3) {
+    const float d_i = p0 - pm, d_i1 = p1 - p0, d_i2 = p2 - p1;
+    const float ml = minmod(d_i, d_i1), mr = minmod(d_i1, d_i2);
+    if (rec == 2) {  // kappa = 1/3: both slopes of a side are the same minmod
+      l = p0 + 0.25f * ((2.f / 3.f) * ml + (4.f / 3.f) * ml);
+      r = p1 - 0.25f * ((2.f / 3.f) * mr + (4.f / 3.f) * mr);
+    } else {
+      l = p0 + 0.5f * ml;
+      r = p1 - 0.5f * mr;
+    }
+  } else {
+    l = p0;
+    r = p1;
+  }
+}
 
-// get(l, q): flux variable l at cell c + q (q = -1..2) of the face between
-// cell c (linear index n) and c + 1 (n + s).
-template <class C, class Src, class Get>
-__device__ __forceinline__ void inviscid_face_r(const Src &S, int64_t n, int d, int64_t s, Get &&get,
-                                                float *fc) {
+// AUSM+/MUSCL flux through the face between cells n and n + s of direction d
+// (f: the quads), and the face's area vector k.
+template <class C>
+__device__ __forceinline__ void inviscid_face(const float4 *__restrict__ f, int64_t sz, int64_t n, int d, int64_t s,
+                                              float *fc, float &k1, float &k2, float &k3) {
   constexpr int NV = C::nv, NS = C::ns;
+  static_assert(C::mix != 0 && NS == 9 && C::turb, "the quads hold nine species and k, omega");
   float pl[NV + 2], pr[NV + 2];
   const int rec = cP.reconstruction;
-  OSTC_UNROLL for (int l = 0; l < NV; ++l) {
-    const float p0 = get(l, 0), p1 = get(l, 1);
+  // the quad's x, y, z, w are flux variables lx, ly, lz, lw (-1: none)
+  auto take = [&](int quad, int lx, int ly, int lz, int lw) {
+    const float4 *q = f + quad * sz + n;
+    const float4 c = __ldg(q), e = __ldg(q + s);
+    float4 m = c, g = e;
     if (rec == 2 || rec == 3) {
-      const float pm = get(l, -1), p2 = get(l, 2);
-      const float d_i = p0 - pm, d_i1 = p1 - p0, d_i2 = p2 - p1;
-      if (rec == 2) {
-        const float neg_l = minmod(d_i, d_i1), pos_l = minmod(d_i1, d_i);
-        const float neg_r = minmod(d_i1, d_i2), pos_r = minmod(d_i2, d_i1);
-        pl[l] = p0 + 0.25f * ((2.f / 3.f) * neg_l + (4.f / 3.f) * pos_l);
-        pr[l] = p1 - 0.25f * ((2.f / 3.f) * pos_r + (4.f / 3.f) * neg_r);
-      } else {
-        pl[l] = p0 + 0.5f * minmod(d_i, d_i1);
-        pr[l] = p1 - 0.5f * minmod(d_i1, d_i2);
-      }
-    } else {
-      pl[l] = p0;
-      pr[l] = p1;
+      m = __ldg(q - s);
+      g = __ldg(q + 2 * s);
     }
-  }
+    if (lx >= 0) reconstruct(rec, m.x, c.x, e.x, g.x, pl[lx], pr[lx]);
+    if (ly >= 0) reconstruct(rec, m.y, c.y, e.y, g.y, pl[ly], pr[ly]);
+    if (lz >= 0) reconstruct(rec, m.z, c.z, e.z, g.z, pl[lz], pr[lz]);
+    if (lw >= 0) reconstruct(rec, m.w, c.w, e.w, g.w, pl[lw], pr[lw]);
+  };
+  take(Quad::rho_vel, 0, 1, 2, 3);
+  take(Quad::p_t_turb, 4, -1, 5 + NS, 6 + NS);
+  take(Quad::y0, 5, 6, 7, 8);
+  take(Quad::y4, 9, 10, 11, 12);
+  take(Quad::y8_mu, 13, -1, -1, -1);
   float el = 0.5f * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]);
   float er = 0.5f * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]);
-  if constexpr (C::mix != 0) {
-    float mwl = 0, mwr = 0;
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-      mwl += pl[5 + l] * cF.mw_inv[l];
-      mwr += pr[5 + l] * cF.mw_inv[l];
-    }
-    const float tl = pl[4] / (pl[0] * kRu * mwl);
-    const float tr = pr[4] / (pr[0] * kRu * mwr);
-    float cpl = 0, cpr = 0, cvl = 0, cvr = 0;
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-      float hl, hr, cpl_l, cpr_l;
-      thermo_one(l, tl, hl, cpl_l);
-      thermo_one(l, tr, hr, cpr_l);
-      cpl += cpl_l * pl[l + 5];
-      cpr += cpr_l * pr[l + 5];
-      cvl += pl[l + 5] * (cpl_l - cF.ru_mw[l]);
-      cvr += pr[l + 5] * (cpr_l - cF.ru_mw[l]);
-      el += hl * pl[l + 5];
-      er += hr * pr[l + 5];
-    }
-    pl[NV] = pl[0] * el - pl[4];
-    pr[NV] = pr[0] * er - pr[4];
-    pl[NV + 1] = cpl / cvl;
-    pr[NV + 1] = cpr / cvr;
-  } else {
-    constexpr float g1 = 1.f / (1.4f - 1.f);
-    pl[NV] = el * pl[0] + pl[4] * g1;
-    pr[NV] = er * pr[0] + pr[4] * g1;
-    pl[NV + 1] = 1.4f;
-    pr[NV + 1] = 1.4f;
+  float mwl = 0, mwr = 0;
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) {
+    mwl += pl[5 + l] * cF.mw_inv[l];
+    mwr += pr[5 + l] * cF.mw_inv[l];
   }
-  const int q0 = 3 * d;
-  const float jl = S.jac(n), jr = S.jac(n + s);
-  const float k1 = 0.5f * (jl * S.metric(q0, n) + jr * S.metric(q0, n + s));
-  const float k2 = 0.5f * (jl * S.metric(q0 + 1, n) + jr * S.metric(q0 + 1, n + s));
-  const float k3 = 0.5f * (jl * S.metric(q0 + 2, n) + jr * S.metric(q0 + 2, n + s));
+  const float tl = pl[4] / (pl[0] * kRu * mwl);
+  const float tr = pr[4] / (pr[0] * kRu * mwr);
+  float cpl = 0, cpr = 0, cvl = 0, cvr = 0;
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) {
+    float hl, hr, cpl_l, cpr_l;
+    thermo_one(l, tl, hl, cpl_l);
+    thermo_one(l, tr, hr, cpr_l);
+    cpl += cpl_l * pl[l + 5];
+    cpr += cpr_l * pr[l + 5];
+    cvl += pl[l + 5] * (cpl_l - cF.ru_mw[l]);
+    cvr += pr[l + 5] * (cpr_l - cF.ru_mw[l]);
+    el += hl * pl[l + 5];
+    er += hr * pr[l + 5];
+  }
+  pl[NV] = pl[0] * el - pl[4];
+  pr[NV] = pr[0] * er - pr[4];
+  pl[NV + 1] = cpl / cvl;
+  pr[NV + 1] = cpr / cvr;
+  const float4 *xi = f + (Quad::metric + d) * sz + n, *jac = f + Quad::metric * sz + n;
+  const float4 ml = __ldg(xi), mr = __ldg(xi + s);
+  const float jl = __ldg(&jac->w), jr = __ldg(&(jac + s)->w);
+  k1 = 0.5f * (jl * ml.x + jr * mr.x);
+  k2 = 0.5f * (jl * ml.y + jr * mr.y);
+  k3 = 0.5f * (jl * ml.z + jr * mr.z);
   const float gk = sqrtf(k1 * k1 + k2 * k2 + k3 * k3);
   const float inv_gk = 1.f / gk;
   const float ul = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) * inv_gk;
@@ -278,124 +251,103 @@ __device__ __forceinline__ void inviscid_face_r(const Src &S, int64_t n, int d, 
   OSTC_UNROLL for (int l = 5; l < NV; ++l) fc[l] = coeff * q(l);
 }
 
-template <class C, class Src>
-__device__ __forceinline__ void inviscid_face_s(const Src &S, int64_t n, int d, int64_t s, float *fc) {
-  inviscid_face_r<C>(S, n, d, s, [&](int l, int q) { return S.prim(l < 5 ? l : l + 1, n + q * s); }, fc);
-}
-
-template <class C>
-__device__ __forceinline__ void inviscid_face(const DevBlock &B, int64_t n, int d, int64_t s, float *fc) {
-  inviscid_face_s<C>(Src64{B}, n, d, s, fc);
-}
-
 // ------------------------------------------------------------- viscous face
-// a(q): the variable at linear index q
-template <class A>
-__device__ __forceinline__ void face_grad(A &&a, int64_t n, int64_t n1, int d, int64_t sx, int64_t sxy, float &dxi,
-                                          float &deta, float &dzeta) {
-  dxi = d == 0 ? a(n1) - a(n) : 0.25f * (a(n + 1) - a(n - 1) + a(n1 + 1) - a(n1 - 1));
-  deta = d == 1 ? a(n1) - a(n) : 0.25f * (a(n + sx) - a(n - sx) + a(n1 + sx) - a(n1 - sx));
-  dzeta = d == 2 ? a(n1) - a(n) : 0.25f * (a(n + sxy) - a(n - sxy) + a(n1 + sxy) - a(n1 - sxy));
+// A quad at both cells of a face and its three computational-space derivatives
+// there (the normal one by the two-point difference, the others by the
+// four-point average).
+struct FaceQuad {
+  float4 a, b, xi, eta, zeta;
+};
+
+__device__ __forceinline__ FaceQuad face_quad(const float4 *__restrict__ q, int64_t s, int d, int64_t sx, int64_t sxy) {
+  FaceQuad r;
+  r.a = __ldg(q);
+  r.b = __ldg(q + s);
+  const float4 normal = make_float4(r.b.x - r.a.x, r.b.y - r.a.y, r.b.z - r.a.z, r.b.w - r.a.w);
+  auto across = [&](int64_t t) {
+    const float4 ap = __ldg(q + t), am = __ldg(q - t), bp = __ldg(q + s + t), bm = __ldg(q + s - t);
+    return make_float4(0.25f * (ap.x - am.x + bp.x - bm.x), 0.25f * (ap.y - am.y + bp.y - bm.y),
+                       0.25f * (ap.z - am.z + bp.z - bm.z), 0.25f * (ap.w - am.w + bp.w - bm.w));
+  };
+  r.xi = d == 0 ? normal : across(1);
+  r.eta = d == 1 ? normal : across(sx);
+  r.zeta = d == 2 ? normal : across(sxy);
+  return r;
 }
 
-// val(v, side): primitive v at cell c (side 0) or c + 1 (side 1) of the face;
-// grad(v, g_xi, g_eta, g_zeta): its computational-space gradient at the face
-// (the face_grad stencil).
-template <class C, class Src, class Val, class Grad>
-__device__ __forceinline__ void viscous_face_r(const Src &S, int64_t n, int d, int64_t s, Val &&val,
-                                               Grad &&grad, float *fv) {
+// Adds the viscous flux through the face between n and n + s (area vector
+// kx, ky, kz) to g.  The derivative of a scalar along k needs the three
+// products k . grad(xi), k . grad(eta), k . grad(zeta) once per face and not the
+// scalar's Cartesian gradient; the species fluxes sum up to their correction.
+template <class C>
+__device__ __forceinline__ void viscous_face_add(const float4 *__restrict__ f, int64_t sz, int64_t sx, int64_t sxy,
+                                                 int64_t n, int d, int64_t s, float kx, float ky, float kz, float *g) {
   constexpr int NS = C::ns;
-  const int64_t n1 = n + s;
-  float mm[9];
-  OSTC_UNROLL for (int q = 0; q < 9; ++q) mm[q] = 0.5f * (S.metric(q, n) + S.metric(q, n1));
-  const float xi_x = mm[0], xi_y = mm[1], xi_z = mm[2], eta_x = mm[3], eta_y = mm[4], eta_z = mm[5];
-  const float zeta_x = mm[6], zeta_y = mm[7], zeta_z = mm[8];
-  auto cart = [&](float a_xi, float a_eta, float a_zeta, float &ax, float &ay, float &az) {
-    ax = a_xi * xi_x + a_eta * eta_x + a_zeta * zeta_x;
-    ay = a_xi * xi_y + a_eta * eta_y + a_zeta * zeta_y;
-    az = a_xi * xi_z + a_eta * eta_z + a_zeta * zeta_z;
+  const float4 *fn = f + n;
+  auto both = [&](int quad) {
+    const float4 a = __ldg(fn + quad * sz), b = __ldg(fn + quad * sz + s);
+    return make_float4(0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z), 0.5f * (a.w + b.w));
   };
-  float g0, g1, g2;
-  float u_x, u_y, u_z, v_x, v_y, v_z, w_x, w_y, w_z, t_x, t_y, t_z;
-  grad(1, g0, g1, g2);
-  cart(g0, g1, g2, u_x, u_y, u_z);
-  grad(2, g0, g1, g2);
-  cart(g0, g1, g2, v_x, v_y, v_z);
-  grad(3, g0, g1, g2);
-  cart(g0, g1, g2, w_x, w_y, w_z);
-  grad(5, g0, g1, g2);
-  cart(g0, g1, g2, t_x, t_y, t_z);
-  const float mul = 0.5f * (S.mul(n) + S.mul(n1));
-  float mut = 0;
-  if constexpr (C::turb) mut = 0.5f * (S.mut(n) + S.mut(n1));
+  const float4 mx = both(Quad::metric), me = both(Quad::metric + 1), mz = both(Quad::metric + 2);
+  const float wall_dist = me.w;
+  const float c_xi = kx * mx.x + ky * mx.y + kz * mx.z, c_eta = kx * me.x + ky * me.y + kz * me.z,
+              c_zeta = kx * mz.x + ky * mz.y + kz * mz.z;
+  // the mean of Y_8, mu, mu_t, lambda comes with Y_8's derivatives, at the end
+  const float4 mu4 = both(Quad::y8_mu), misc = both(Quad::misc);
+  const float mul = mu4.y, mut = mu4.z, conductivity = mu4.w + misc.x;
   const float viscosity = mul + mut;
   constexpr float third = 1.f / 3.f;
-  float tau_xx = viscosity * (4 * u_x - 2 * v_y - 2 * w_z) * third;
-  float tau_yy = viscosity * (4 * v_y - 2 * u_x - 2 * w_z) * third;
-  float tau_zz = viscosity * (4 * w_z - 2 * u_x - 2 * v_y) * third;
-  const float tau_xy = viscosity * (u_y + v_x);
-  const float tau_xz = viscosity * (u_z + w_x);
-  const float tau_yz = viscosity * (v_z + w_y);
-  if constexpr (C::turb) {
-    const float tt = -(1.f / 3.f) * (val(0, 0) * val(6 + NS, 0) + val(0, 1) * val(6 + NS, 1));
-    tau_xx += tt;
-    tau_yy += tt;
-    tau_zz += tt;
+  float rhom, rho_a, rho_b;
+  {
+    const FaceQuad q = face_quad(fn + Quad::rho_vel * sz, s, d, sx, sxy);
+    auto cart = [&](float a_xi, float a_eta, float a_zeta, float &ax, float &ay, float &az) {
+      ax = a_xi * mx.x + a_eta * me.x + a_zeta * mz.x;
+      ay = a_xi * mx.y + a_eta * me.y + a_zeta * mz.y;
+      az = a_xi * mx.z + a_eta * me.z + a_zeta * mz.z;
+    };
+    float u_x, u_y, u_z, v_x, v_y, v_z, w_x, w_y, w_z;
+    cart(q.xi.y, q.eta.y, q.zeta.y, u_x, u_y, u_z);
+    cart(q.xi.z, q.eta.z, q.zeta.z, v_x, v_y, v_z);
+    cart(q.xi.w, q.eta.w, q.zeta.w, w_x, w_y, w_z);
+    const float4 ta = __ldg(fn + Quad::p_t_turb * sz), tb = __ldg(fn + Quad::p_t_turb * sz + s);
+    const float tt = -third * (q.a.x * ta.z + q.b.x * tb.z);  // -2/3 rho k
+    const float tau_xx = viscosity * (4 * u_x - 2 * v_y - 2 * w_z) * third + tt;
+    const float tau_yy = viscosity * (4 * v_y - 2 * u_x - 2 * w_z) * third + tt;
+    const float tau_zz = viscosity * (4 * w_z - 2 * u_x - 2 * v_y) * third + tt;
+    const float tau_xy = viscosity * (u_y + v_x);
+    const float tau_xz = viscosity * (u_z + w_x);
+    const float tau_yz = viscosity * (v_z + w_y);
+    const float f1 = kx * tau_xx + ky * tau_xy + kz * tau_xz, f2 = kx * tau_xy + ky * tau_yy + kz * tau_yz,
+                f3 = kx * tau_xz + ky * tau_yz + kz * tau_zz;
+    g[1] += f1;
+    g[2] += f2;
+    g[3] += f3;
+    g[4] += 0.5f * (q.a.y + q.b.y) * f1 + 0.5f * (q.a.z + q.b.z) * f2 + 0.5f * (q.a.w + q.b.w) * f3;
+    rho_a = q.a.x;
+    rho_b = q.b.x;
+    rhom = 0.5f * (rho_a + rho_b);
   }
-  const int q0 = 3 * d;
-  const float ja = S.jac(n), jb = S.jac(n1);
-  const float kx = 0.5f * (S.metric(q0, n) * ja + S.metric(q0, n1) * jb);
-  const float ky = 0.5f * (S.metric(q0 + 1, n) * ja + S.metric(q0 + 1, n1) * jb);
-  const float kz = 0.5f * (S.metric(q0 + 2, n) * ja + S.metric(q0 + 2, n1) * jb);
-  fv[0] = 0;
-  fv[1] = kx * tau_xx + ky * tau_xy + kz * tau_xz;
-  fv[2] = kx * tau_xy + ky * tau_yy + kz * tau_yz;
-  fv[3] = kx * tau_xz + ky * tau_yz + kz * tau_zz;
-  const float um = 0.5f * (val(1, 0) + val(1, 1));
-  const float vm = 0.5f * (val(2, 0) + val(2, 1));
-  const float wm = 0.5f * (val(3, 0) + val(3, 1));
-  float conductivity = 0.5f * (S.cond(n) + S.cond(n1));
-  if constexpr (C::turb) conductivity += 0.5f * (S.tcond(n) + S.tcond(n1));
-  fv[4] = um * fv[1] + vm * fv[2] + wm * fv[3] + conductivity * (kx * t_x + ky * t_y + kz * t_z);
-  if constexpr (C::mix != 0) {
-    float turb_d = 0;
-    if constexpr (C::turb) turb_d = mut / cF.Sct;
-    const float tm = 0.5f * (val(5, 0) + val(5, 1));
-    float rho_uc = 0, rho_vc = 0, rho_wc = 0, hflux = 0;
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-      const float dif = 0.5f * (S.rho_d(l, n) + S.rho_d(l, n1)) + turb_d;
-      float yx, yy, yz, h, cp_unused;
-      grad(6 + l, g0, g1, g2);
-      cart(g0, g1, g2, yx, yy, yz);
-      thermo_one(l, tm, h, cp_unused);
-      // the diffusive flux of species l through the face, before the correction
-      fv[5 + l] = dif * (kx * yx + ky * yy + kz * yz);
-      hflux += h * fv[5 + l];
-      rho_uc += dif * yx;
-      rho_vc += dif * yy;
-      rho_wc += dif * yz;
-    }
-    fv[4] += hflux;
-    const float corr = kx * rho_uc + ky * rho_vc + kz * rho_wc;
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) fv[5 + l] -= 0.5f * (val(6 + l, 0) + val(6 + l, 1)) * corr;
-  }
-  if constexpr (C::turb) {
-    float k_x, k_y, k_z, o_x, o_y, o_z;
-    grad(6 + NS, g0, g1, g2);
-    cart(g0, g1, g2, k_x, k_y, k_z);
-    grad(7 + NS, g0, g1, g2);
-    cart(g0, g1, g2, o_x, o_y, o_z);
-    const float wall_dist = 0.5f * (S.wall(n) + S.wall(n1));
+  float tm;
+  {
+    const FaceQuad q = face_quad(fn + Quad::p_t_turb * sz, s, d, sx, sxy);
+    tm = 0.5f * (q.a.y + q.b.y);
+    g[4] += conductivity * (c_xi * q.xi.y + c_eta * q.eta.y + c_zeta * q.zeta.y);
+    const float k_n = c_xi * q.xi.z + c_eta * q.eta.z + c_zeta * q.zeta.z;
+    const float o_n = c_xi * q.xi.w + c_eta * q.eta.w + c_zeta * q.zeta.w;
     float f1 = 1;
     if (wall_dist > 1e-25f) {
-      const float km = 0.5f * (val(6 + NS, 0) + val(6 + NS, 1));
-      const float omegam = 0.5f * (val(7 + NS, 0) + val(7 + NS, 1));
+      auto dx = [&](float a, float b, float c) { return a * mx.x + b * me.x + c * mz.x; };
+      auto dy = [&](float a, float b, float c) { return a * mx.y + b * me.y + c * mz.y; };
+      auto dz = [&](float a, float b, float c) { return a * mx.z + b * me.z + c * mz.z; };
+      const float cross = dx(q.xi.z, q.eta.z, q.zeta.z) * dx(q.xi.w, q.eta.w, q.zeta.w) +
+                          dy(q.xi.z, q.eta.z, q.zeta.z) * dy(q.xi.w, q.eta.w, q.zeta.w) +
+                          dz(q.xi.z, q.eta.z, q.zeta.z) * dz(q.xi.w, q.eta.w, q.zeta.w);
+      const float km = 0.5f * (q.a.z + q.b.z), omegam = 0.5f * (q.a.w + q.b.w);
       const float param1 = sqrtf(km) / (0.09f * omegam * wall_dist);
-      const float rhom = 0.5f * (val(0, 0) + val(0, 1));
       const float d2 = wall_dist * wall_dist;
       const float param2 = 500 * mul / (rhom * d2 * omegam);
       constexpr float so2 = static_cast<float>(sst::sigma_omega2);
-      const float CDkomega = fmaxf(1e-20f, 2 * rhom * so2 / omegam * (k_x * o_x + k_y * o_y + k_z * o_z));
+      const float CDkomega = fmaxf(1e-20f, 2 * rhom * so2 / omegam * cross);
       const float param3 = 4 * rhom * so2 * km / (CDkomega * d2);
       const float arg1 = fminf(fmaxf(param1, param2), param3);
       f1 = tanh_pos(arg1 * arg1 * arg1 * arg1);
@@ -403,26 +355,54 @@ __device__ __forceinline__ void viscous_face_r(const Src &S, int64_t n, int d, i
     const float sigma_k = static_cast<float>(sst::sigma_k2) + static_cast<float>(sst::delta_sigma_k) * f1;
     const float sigma_omega =
         static_cast<float>(sst::sigma_omega2) + static_cast<float>(sst::delta_sigma_omega) * f1;
-    fv[5 + NS] = (mul + mut * sigma_k) * (kx * k_x + ky * k_y + kz * k_z);
-    fv[6 + NS] = (mul + mut * sigma_omega) * (kx * o_x + ky * o_y + kz * o_z);
+    g[5 + NS] += (mul + mut * sigma_k) * k_n;
+    g[6 + NS] += (mul + mut * sigma_omega) * o_n;
   }
-}
-
-template <class C, class Src>
-__device__ __forceinline__ void viscous_face_s(const Src &S, int64_t sx, int64_t sxy, int64_t n, int d, int64_t s,
-                                               float *fv) {
-  const int64_t n1 = n + s;
-  viscous_face_r<C>(
-      S, n, d, s, [&](int v, int side) { return S.prim(v, side ? n1 : n); },
-      [&](int v, float &g0, float &g1, float &g2) {
-        face_grad([&](int64_t q) { return S.prim(v, q); }, n, n1, d, sx, sxy, g0, g1, g2);
-      },
-      fv);
-}
-
-template <class C>
-__device__ __forceinline__ void viscous_face(const DevBlock &B, int64_t n, int d, int64_t s, float *fv) {
-  viscous_face_s<C>(Src64{B}, B.G.sx, B.G.sxy, n, d, s, fv);
+  const float turb_d = mut / cF.Sct;
+  float hflux = 0, total = 0;
+  auto species = [&](int l, float dif, float xi, float eta, float zeta) {
+    float h, cp_unused;
+    thermo_one(l, tm, h, cp_unused);
+    const float flux = (dif + turb_d) * (c_xi * xi + c_eta * eta + c_zeta * zeta);
+    g[5 + l] += flux;
+    hflux += h * flux;
+    total += flux;
+  };
+  float4 y0, y4;
+  float y8;
+  {
+    const float4 dif = both(Quad::d0);
+    const FaceQuad q = face_quad(fn + Quad::y0 * sz, s, d, sx, sxy);
+    species(0, dif.x, q.xi.x, q.eta.x, q.zeta.x);
+    species(1, dif.y, q.xi.y, q.eta.y, q.zeta.y);
+    species(2, dif.z, q.xi.z, q.eta.z, q.zeta.z);
+    species(3, dif.w, q.xi.w, q.eta.w, q.zeta.w);
+    y0 = make_float4(0.5f * (q.a.x + q.b.x), 0.5f * (q.a.y + q.b.y), 0.5f * (q.a.z + q.b.z), 0.5f * (q.a.w + q.b.w));
+  }
+  {
+    const float4 dif = both(Quad::d4);
+    const FaceQuad q = face_quad(fn + Quad::y4 * sz, s, d, sx, sxy);
+    species(4, dif.x, q.xi.x, q.eta.x, q.zeta.x);
+    species(5, dif.y, q.xi.y, q.eta.y, q.zeta.y);
+    species(6, dif.z, q.xi.z, q.eta.z, q.zeta.z);
+    species(7, dif.w, q.xi.w, q.eta.w, q.zeta.w);
+    y4 = make_float4(0.5f * (q.a.x + q.b.x), 0.5f * (q.a.y + q.b.y), 0.5f * (q.a.z + q.b.z), 0.5f * (q.a.w + q.b.w));
+  }
+  {
+    const FaceQuad q = face_quad(fn + Quad::y8_mu * sz, s, d, sx, sxy);
+    species(8, misc.w, q.xi.x, q.eta.x, q.zeta.x);
+    y8 = 0.5f * (q.a.x + q.b.x);
+  }
+  g[4] += hflux;
+  g[5] -= y0.x * total;
+  g[6] -= y0.y * total;
+  g[7] -= y0.z * total;
+  g[8] -= y0.w * total;
+  g[9] -= y4.x * total;
+  g[10] -= y4.y * total;
+  g[11] -= y4.z * total;
+  g[12] -= y4.w * total;
+  g[13] -= y8 * total;
 }
 
 // ------------------------------------------------------------- SST source
@@ -628,35 +608,27 @@ __global__ void __launch_bounds__(kCta, 4) k_chem_list(const DevBlock *__restric
 // Local time step of cell (i, j, k) in FP32 (local_time_step,
 // src/TimeAdvanceFunc.cuh:21-71); also stores the spectral radii the DPLUR
 // sweeps use.
-template <class C, class Src>
-__device__ __forceinline__ void local_time_step_s(const DevBlock &B, const Src &S, int i, int j, int k, int64_t n,
-                                                  int64_t nd) {
-  const int64_t szd = B.D.size;
+template <class C>
+__device__ __forceinline__ void local_time_step_q(const DevBlock &B, const float4 *__restrict__ f, int i, int j, int k,
+                                                  int64_t n, int64_t nd) {
+  using Q = fp32::Quad;
+  const int64_t szd = B.D.size, sz = B.G.size;
   const bool three_d = B.mz > 1;
-  const float m11 = S.metric(0, n), m12 = S.metric(1, n), m13 = S.metric(2, n);
-  const float m21 = S.metric(3, n), m22 = S.metric(4, n), m23 = S.metric(5, n);
-  const float m31 = S.metric(6, n), m32 = S.metric(7, n), m33 = S.metric(8, n);
-  const float grad_xi = sqrtf(m11 * m11 + m12 * m12 + m13 * m13);
-  const float grad_eta = sqrtf(m21 * m21 + m22 * m22 + m23 * m23);
-  const float grad_zeta = sqrtf(m31 * m31 + m32 * m32 + m33 * m33);
-  const float u = S.prim(1, n), v = S.prim(2, n), w = S.prim(3, n);
-  const float a = S.acoustic(n);
-  const float s0 = fabsf(u * m11 + v * m12 + w * m13) + a * grad_xi;
-  const float s1 = fabsf(u * m21 + v * m22 + w * m23) + a * grad_eta;
-  const float s2 = three_d ? fabsf(u * m31 + v * m32 + w * m33) + a * grad_zeta : 0.f;
+  const float4 m1 = __ldg(f + Q::metric * sz + n), m2 = __ldg(f + (Q::metric + 1) * sz + n),
+               m3 = __ldg(f + (Q::metric + 2) * sz + n), s = __ldg(f + Q::rho_vel * sz + n),
+               misc = __ldg(f + Q::misc * sz + n), mu = __ldg(f + Q::y8_mu * sz + n);
+  const float grad_xi = sqrtf(m1.x * m1.x + m1.y * m1.y + m1.z * m1.z);
+  const float grad_eta = sqrtf(m2.x * m2.x + m2.y * m2.y + m2.z * m2.z);
+  const float grad_zeta = sqrtf(m3.x * m3.x + m3.y * m3.y + m3.z * m3.z);
+  const float a = misc.y;
+  const float s0 = fabsf(s.y * m1.x + s.z * m1.y + s.w * m1.z) + a * grad_xi;
+  const float s1 = fabsf(s.y * m2.x + s.z * m2.y + s.w * m2.z) + a * grad_eta;
+  const float s2 = three_d ? fabsf(s.y * m3.x + s.z * m3.y + s.w * m3.z) + a * grad_zeta : 0.f;
   B.inv_spec[nd] = s0;
   B.inv_spec[szd + nd] = s1;
   B.inv_spec[2 * szd + nd] = s2;
-  if (B.inv_spec32) {
-    B.inv_spec32[nd] = s0;
-    B.inv_spec32[szd + nd] = s1;
-    B.inv_spec32[2 * szd + nd] = s2;
-  }
-  float gamma = 1.4f;
-  if constexpr (C::mix != 0) gamma = S.gamma(n);
-  const float coeff_1 = fmaxf(gamma, 4.f / 3.f) / S.prim(0, n);
-  float coeff_2 = S.mul(n) / cF.Pr;
-  if constexpr (C::turb) coeff_2 += S.mut(n) / cF.Prt;
+  const float coeff_1 = fmaxf(misc.z, 4.f / 3.f) / s.x;
+  const float coeff_2 = mu.y / cF.Pr + mu.z / cF.Prt;
   float srv = grad_xi * grad_xi + grad_eta * grad_eta;
   if (three_d) srv += grad_zeta * grad_zeta;
   srv *= coeff_1 * coeff_2;
@@ -724,14 +696,11 @@ __device__ __forceinline__ void dir_tile(const Tiles &T, int &b, int &t0, int &t
 template <class C>
 __device__ __forceinline__ void face_g(const DevBlock &B, int64_t nl, int d, int64_t s, float *g) {
   constexpr int NV = C::nv;
-  const fp32::Src32<C> S{B.f32, B.G.size};
-  fp32::inviscid_face_s<C>(S, nl, d, s, g);
+  float kx, ky, kz;
+  fp32::inviscid_face<C>(B.f32, B.G.size, nl, d, s, g, kx, ky, kz);
   OSTC_UNROLL for (int l = 0; l < NV; ++l) g[l] = -g[l];
-  if (cP.viscous_order != 0) {
-    float t[NV];
-    fp32::viscous_face_s<C>(S, B.G.sx, B.G.sxy, nl, d, s, t);
-    OSTC_UNROLL for (int l = 0; l < NV; ++l) g[l] += t[l];
-  }
+  if (cP.viscous_order != 0)
+    fp32::viscous_face_add<C>(B.f32, B.G.size, B.G.sx, B.G.sxy, nl, d, s, kx, ky, kz, g);
 }
 
 // The FP32 copy of the operands of the direction passes, over every point of
@@ -739,49 +708,54 @@ __device__ __forceinline__ void face_g(const DevBlock &B, int64_t nl, int d, int
 // writes mu_t and lambda_t) ...
 template <class C>
 __global__ void __launch_bounds__(256) k_pack32(const DevBlock *__restrict__ blks, int b) {
-  using L = fp32::F32<C>;
+  using Q = fp32::Quad;
   const DevBlock &B = blks[b];
   const int64_t sz = B.G.size;
-  float *f = B.f32;
+  float4 *f = B.f32;
   for (int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; n < sz;
        n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     // all loads, then all stores (a store would otherwise hold back the
     // loads after it: the compiler cannot rule out that they overlap)
-    float v[L::n_dynamic];
-    OSTC_UNROLL for (int q = 0; q < L::n_dynamic; ++q) v[q] = 0.f;
-    OSTC_UNROLL for (int q = 0; q < 6; ++q) v[L::prim + q] = static_cast<float>(__ldg(B.bv + q * sz + n));
-    OSTC_UNROLL for (int q = 0; q < C::nsc; ++q) v[L::prim + 6 + q] = static_cast<float>(__ldg(B.sv + q * sz + n));
-    v[L::mul] = static_cast<float>(__ldg(B.mul + n));
-    v[L::cond] = static_cast<float>(__ldg(B.cond + n));
-    if constexpr (C::turb) {
-      v[L::mut] = static_cast<float>(__ldg(B.mut + n));
-      v[L::tcond] = static_cast<float>(__ldg(B.turb_cond + n));
+    float v[4 * Q::n_dynamic];
+    auto bv = [&](int l) { return fp32::ldf(B.bv + l * sz + n); };
+    auto sv = [&](int l) { return fp32::ldf(B.sv + l * sz + n); };
+    OSTC_UNROLL for (int l = 0; l < 4; ++l) {
+      v[4 * Q::rho_vel + l] = bv(l);
+      v[4 * Q::y0 + l] = sv(l);
+      v[4 * Q::y4 + l] = sv(4 + l);
+      v[4 * Q::d0 + l] = fp32::ldf(B.rho_d + l * sz + n);
+      v[4 * Q::d4 + l] = fp32::ldf(B.rho_d + (4 + l) * sz + n);
     }
-    OSTC_UNROLL for (int l = 0; l < C::ns; ++l) v[L::rho_d + l] = static_cast<float>(__ldg(B.rho_d + l * sz + n));
-    v[L::acoustic] = static_cast<float>(__ldg(B.acoustic + n));
-    if constexpr (C::mix != 0) v[L::gamma] = static_cast<float>(__ldg(B.gamma + n));
-    OSTC_UNROLL for (int q = 0; q < L::n_dynamic; ++q) {
-      if (q == L::mut || q == L::tcond) {
-        if constexpr (!C::turb) continue;
-      }
-      if (q == L::gamma && C::mix == 0) continue;
-      f[q * sz + n] = v[q];
-    }
+    v[4 * Q::p_t_turb] = bv(4);
+    v[4 * Q::p_t_turb + 1] = bv(5);
+    v[4 * Q::p_t_turb + 2] = sv(C::ns);
+    v[4 * Q::p_t_turb + 3] = sv(C::ns + 1);
+    v[4 * Q::y8_mu] = sv(8);
+    v[4 * Q::y8_mu + 1] = fp32::ldf(B.mul + n);
+    v[4 * Q::y8_mu + 2] = fp32::ldf(B.mut + n);
+    v[4 * Q::y8_mu + 3] = fp32::ldf(B.cond + n);
+    v[4 * Q::misc] = fp32::ldf(B.turb_cond + n);
+    v[4 * Q::misc + 1] = fp32::ldf(B.acoustic + n);
+    v[4 * Q::misc + 2] = fp32::ldf(B.gamma + n);
+    v[4 * Q::misc + 3] = fp32::ldf(B.rho_d + 8 * sz + n);
+    OSTC_UNROLL for (int q = 0; q < Q::n_dynamic; ++q)
+      f[q * sz + n] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
   }
 }
 
 // ... and the geometry, which changes only when the grid is set.
 template <class C>
 __global__ void __launch_bounds__(256) k_pack32_static(const DevBlock *__restrict__ blks, int b) {
-  using L = fp32::F32<C>;
+  using Q = fp32::Quad;
   const DevBlock &B = blks[b];
   const int64_t sz = B.G.size;
-  float *f = B.f32;
   for (int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; n < sz;
        n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    f[L::wall * sz + n] = B.wall_dist ? static_cast<float>(B.wall_dist[n]) : 0.f;
-    f[L::jac * sz + n] = static_cast<float>(B.jac[n]);
-    OSTC_UNROLL for (int q = 0; q < 9; ++q) f[(L::metric + q) * sz + n] = static_cast<float>(B.metric[q * sz + n]);
+    const float extra[3] = {static_cast<float>(B.jac[n]), B.wall_dist ? static_cast<float>(B.wall_dist[n]) : 0.f, 0.f};
+    OSTC_UNROLL for (int d = 0; d < 3; ++d) {
+      auto m = [&](int q) { return static_cast<float>(B.metric[(3 * d + q) * sz + n]); };
+      B.f32[(Q::metric + d) * sz + n] = make_float4(m(0), m(1), m(2), extra[d]);
+    }
   }
 }
 
@@ -809,7 +783,7 @@ __global__ void __launch_bounds__(kCta, MINB) k_flux_x(const DevBlock *__restric
     const float gm = __shfl_up_sync(0xffffffffu, g[l], 1);
     if (cell) B.dq[l * szd + nd] += static_cast<double>(g[l] - gm);
   }
-  if (cell) local_time_step_s<C>(B, fp32::Src32<C>{B.f32, B.G.size}, f, j, k, B.G.at(f, j, k), nd);
+  if (cell) local_time_step_q<C>(B, B.f32, f, j, k, B.G.at(f, j, k), nd);
 }
 
 template <class C, int D, int MINB>
@@ -843,6 +817,67 @@ __global__ void __launch_bounds__(kCta, MINB) k_flux_march(const DevBlock *__res
   }
 }
 
+// The terms of a cell's flux-Jacobian product that no direction enters
+// (compute_jacobian_times_dq, src/DPLURHPP.cuh:78-125), kept per cell so that a
+// sweep does not sum over the species for each of the six neighbours that take
+// them: once per step the total enthalpy h (beside the spectral radii, radii32)
+// and the weights gamma R T / W_l - (gamma - 1) h_l of the species increments
+// in the pressure term, and per sweep the pressure term itself, by the kernel
+// that writes the increments.
+template <class C>
+__device__ __forceinline__ float pressure_term32(const DevBlock &B, int64_t n, int64_t nd, const float *d) {
+  const int64_t szd = B.D.size;
+  const float4 s = __ldg(B.f32 + fp32::Quad::rho_vel * B.G.size + n);
+  const float gamma = __ldg(&(B.f32 + fp32::Quad::misc * B.G.size + n)->z);
+  float p = (gamma - 1) * (0.5f * (s.y * s.y + s.z * s.z + s.w * s.w) * d[0] - s.y * d[1] - s.z * d[2] - s.w * d[3] + d[4]);
+  OSTC_UNROLL for (int l = 0; l < C::ns; ++l) p += B.weight32[l * szd + nd] * d[5 + l];
+  return p;
+}
+
+// increments of a cell in buffer q of the sweeps: four quads in the order of
+// the flux variables
+template <class C>
+__device__ __forceinline__ void store_increments32(float4 *f, int64_t szd, int64_t nd, const float *d) {
+  static_assert(C::nv == 16, "four quads");
+  OSTC_UNROLL for (int q = 0; q < 4; ++q) f[q * szd + nd] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
+}
+template <class C>
+__device__ __forceinline__ void load_increments32(const float4 *__restrict__ f, int64_t szd, int64_t nd, float *d) {
+  OSTC_UNROLL for (int q = 0; q < 4; ++q) {
+    const float4 v = __ldg(f + q * szd + nd);
+    d[4 * q] = v.x;
+    d[4 * q + 1] = v.y;
+    d[4 * q + 2] = v.z;
+    d[4 * q + 3] = v.w;
+  }
+}
+
+// of dq0, by k_sweep_terms
+template <class C>
+__device__ __forceinline__ void sweep_terms32(const DevBlock &B, int64_t n, int64_t nd) {
+  constexpr int NS = C::ns, NV = C::nv;
+  const int64_t sz = B.G.size, szd = B.D.size;
+  const float4 s = __ldg(B.f32 + fp32::Quad::rho_vel * sz + n);
+  const double t = ld(B.bv + 5 * sz + n), gamma = ld(B.gamma + n);
+  float d[NV];
+  load_increments32<C>(B.dqf[0], szd, nd, d);
+  double hk[NS], h = 0.5 * (s.y * s.y + s.z * s.z + s.w * s.w);
+  enthalpy<NS>(t, hk);
+  const float g1 = static_cast<float>(gamma) - 1;
+  float p = g1 * (0.5f * (s.y * s.y + s.z * s.z + s.w * s.w) * d[0] - s.y * d[1] - s.z * d[2] - s.w * d[3] + d[4]);
+  float w[NS];
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) {
+    h += ld(B.sv + l * sz + n) * hk[l];
+    w[l] = static_cast<float>(gamma * t * cP.ru_mw[l] - (gamma - 1) * hk[l]);
+    p += w[l] * d[5 + l];
+  }
+  const float4 radii = make_float4(static_cast<float>(ld(B.inv_spec + nd)), static_cast<float>(ld(B.inv_spec + szd + nd)),
+                                   static_cast<float>(ld(B.inv_spec + 2 * szd + nd)), static_cast<float>(h));
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) B.weight32[l * szd + nd] = w[l];
+  B.radii32[nd] = radii;
+  B.terms32[nd] = p;
+}
+
 // EPI solve of a DPLUR sweep with the stored factors of the leading NA x NA
 // block; the trailing species have the single pivot diag, so their solve is
 // rhs / diag, the operation the full factors would do for them.
@@ -863,19 +898,17 @@ template <class C>
 __global__ void __launch_bounds__(kCta, 4) k_sweep_mx(const DevBlock *__restrict__ blks, Tiles T, int in_sel,
                                                       int out_sel) {
   constexpr int NS = C::ns, NV = C::nv;
-  using fp32::ldf;
   int b, i, j, k;
   if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
   const DevBlock &B = blks[b];
-  const float *dqin = B.dqf[in_sel];
-  const float *dq0 = B.dqf[0];
+  using Q = fp32::Quad;
+  const float4 *dqin = B.dqf[in_sel];
   const int64_t sz = B.G.size, szd = B.D.size, sz0 = B.Z.size;
   const int64_t n = B.G.at(i, j, k), nd = B.D.at(i, j, k), nz = B.Z.at(i, j, k);
   const int64_t sx = B.G.sx, sxy = B.G.sxy, dsx = B.D.sx, dsxy = B.D.sxy;
-  const fp32::Src32<C> f{B.f32, sz};
+  const float4 *f = B.f32;
   float tot[NV];
   OSTC_UNROLL for (int l = 0; l < NV; ++l) tot[l] = 0;
-  const float *isr = B.inv_spec32;  // FP32 values, as k_flux_x computed them
 #pragma unroll 1
   for (int q = 0; q < 6; ++q) {
     const int dir = q < 3 ? q : q - 3;
@@ -885,55 +918,43 @@ __global__ void __launch_bounds__(kCta, 4) k_sweep_mx(const DevBlock *__restrict
     if (plus ? id == ext - 1 : id == 0) continue;
     const int64_t gs = dir == 0 ? 1 : (dir == 1 ? sx : sxy), ds = dir == 0 ? 1 : (dir == 1 ? dsx : dsxy);
     const int64_t on = plus ? n + gs : n - gs, od = plus ? nd + ds : nd - ds;
-    const float sr = __ldg(isr + dir * szd + od);
     // compute_jacobian_times_dq (src/DPLURHPP.cuh:78-125) at the neighbour,
     // its state from the step's FP32 copy (k_pack32; unchanged until the update)
-    const float xi_x = f.metric(3 * dir, on), xi_y = f.metric(3 * dir + 1, on), xi_z = f.metric(3 * dir + 2, on);
-    const float u = f.prim(1, on), v = f.prim(2, on), w = f.prim(3, on);
-    const float U = xi_x * u + xi_y * v + xi_z * w;
-    const float lmd1 = U + (plus ? -sr : sr);
-    const float e = 0.5f * (u * u + v * v + w * w);
+    const float4 xi = __ldg(f + (Q::metric + dir) * sz + on), vel = __ldg(f + Q::rho_vel * sz + on);
+    const float4 y0 = __ldg(f + Q::y0 * sz + on), y4 = __ldg(f + Q::y4 * sz + on);
+    const float4 turb = __ldg(f + Q::p_t_turb * sz + on), radii = __ldg(B.radii32 + od);
+    const float y8 = __ldg(&(f + Q::y8_mu * sz + on)->x);
+    const float p = __ldg(B.terms32 + in_sel * szd + od), h = radii.w;
     float d[NV];
-    OSTC_UNROLL for (int l = 0; l < NV; ++l) d[l] = __ldg(dqin + l * szd + od);
-    float gamma = 1.4f, b3 = 0, b4 = 0, h = 0;
-    if constexpr (C::mix != 0) {
-      const float t = f.prim(5, on);
-      gamma = f.gamma(on);
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-        const float hk = __ldg(B.h_spec32 + l * szd + od);
-        b3 += fp32::kRu * t * cF.mw_inv[l] * d[5 + l];
-        b4 += hk * d[5 + l];
-        h += f.prim(6 + l, on) * hk;
-      }
-      b3 *= gamma;
-      b4 *= gamma - 1;
-      h += e;
-    } else {
-      h = gamma / (gamma - 1) * f.prim(4, on) / f.prim(0, on) + e;
-    }
-    const float b1 = xi_x * d[1] + xi_y * d[2] + xi_z * d[3] - U * d[0];
-    const float b2 = (gamma - 1) * (e * d[0] - u * d[1] - v * d[2] - w * d[3] + d[4]);
-    const float b34 = b3 - b4;
+    load_increments32<C>(dqin, szd, od, d);
+    const float sr = dir == 0 ? radii.x : (dir == 1 ? radii.y : radii.z);
+    const float U = xi.x * vel.y + xi.y * vel.z + xi.z * vel.w;
+    const float b1 = xi.x * d[1] + xi.y * d[2] + xi.z * d[3] - U * d[0];
     const float sg = plus ? -0.5f : 0.5f;
-    tot[0] += sg * (b1 + lmd1 * d[0]);
-    tot[1] += sg * (u * b1 + xi_x * b2 + lmd1 * d[1] + xi_x * b34);
-    tot[2] += sg * (v * b1 + xi_y * b2 + lmd1 * d[2] + xi_y * b34);
-    tot[3] += sg * (w * b1 + xi_z * b2 + lmd1 * d[3] + xi_z * b34);
-    tot[4] += sg * (h * b1 + U * b2 + lmd1 * d[4] + U * b34);
-    OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) tot[5 + l] += sg * (lmd1 * d[5 + l] + f.prim(6 + l, on) * b1);
+    const float lmd1 = sg * (U + (plus ? -sr : sr)), c1 = sg * b1, cp = sg * p;
+    tot[0] += c1 + lmd1 * d[0];
+    tot[1] += vel.y * c1 + xi.x * cp + lmd1 * d[1];
+    tot[2] += vel.z * c1 + xi.y * cp + lmd1 * d[2];
+    tot[3] += vel.w * c1 + xi.z * cp + lmd1 * d[3];
+    tot[4] += h * c1 + U * cp + lmd1 * d[4];
+    const float y[NV - 5] = {y0.x, y0.y, y0.z, y0.w, y4.x, y4.y, y4.z, y4.w, y8, turb.z, turb.w};
+    OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) tot[5 + l] += lmd1 * d[5 + l] + y[l] * c1;
   }
+  const float4 rad = __ldg(B.radii32 + nd);
+  float dq0[NV];
+  load_increments32<C>(B.dqf[0], szd, nd, dq0);
   const double dt = B.dt_local[nz];
-  const double diag = 1 + dt * (static_cast<double>(isr[nd]) + static_cast<double>(isr[szd + nd]) +
-                                static_cast<double>(isr[2 * szd + nd]));
+  const double diag =
+      1 + dt * (static_cast<double>(rad.x) + static_cast<double>(rad.y) + static_cast<double>(rad.z));
   double out[NV];
   if constexpr (C::mix != 2) {
-    OSTC_UNROLL for (int l = 0; l < 5 + NS; ++l) out[l] = static_cast<double>(dq0[l * szd + nd]) + dt * tot[l] / diag;
+    OSTC_UNROLL for (int l = 0; l < 5 + NS; ++l) out[l] = static_cast<double>(dq0[l]) + dt * tot[l] / diag;
   } else {
-    OSTC_UNROLL for (int l = 0; l < 5; ++l) out[l] = static_cast<double>(dq0[l * szd + nd]) + dt * tot[l] / diag;
+    OSTC_UNROLL for (int l = 0; l < 5; ++l) out[l] = static_cast<double>(dq0[l]) + dt * tot[l] / diag;
     const int method = cP.chem_src_method;
     if (B.chem_quiet && B.chem_quiet[nz]) {
       // chemically quiet: the stored factors would be diag I
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[(5 + l) * szd + nd]) + dt * tot[5 + l] / diag;
+      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[5 + l]) + dt * tot[5 + l] / diag;
     } else if (method == 1) {
       double rhs[NS];
       OSTC_UNROLL for (int l = 0; l < NS; ++l) rhs[l] = static_cast<double>(tot[5 + l]) * dt;
@@ -941,28 +962,30 @@ __global__ void __launch_bounds__(kCta, 4) k_sweep_mx(const DevBlock *__restrict
         epi_solve_block<NS, NS - 1>(B, nz, sz0, diag, rhs);
       else
         epi_solve_block<NS, NS>(B, nz, sz0, diag, rhs);
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[(5 + l) * szd + nd]) + rhs[l];
+      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[5 + l]) + rhs[l];
     } else if (method == 2) {
       OSTC_UNROLL for (int l = 0; l < NS; ++l)
-        out[5 + l] = static_cast<double>(dq0[(5 + l) * szd + nd]) + dt * tot[5 + l] / (diag - dt * B.chem_jac[l * sz0 + nz]);
+        out[5 + l] = static_cast<double>(dq0[5 + l]) + dt * tot[5 + l] / (diag - dt * B.chem_jac[l * sz0 + nz]);
     } else {
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[(5 + l) * szd + nd]) + dt * tot[5 + l] / diag;
+      OSTC_UNROLL for (int l = 0; l < NS; ++l) out[5 + l] = static_cast<double>(dq0[5 + l]) + dt * tot[5 + l] / diag;
     }
   }
   if constexpr (C::turb) {
     if (cP.turb_implicit == 1) {
-      out[NS + 5] = static_cast<double>(dq0[(NS + 5) * szd + nd]) + dt * tot[5 + NS] / (diag - dt * B.turb_src_jac[nz]);
-      out[NS + 6] = static_cast<double>(dq0[(NS + 6) * szd + nd]) + dt * tot[6 + NS] / (diag - dt * B.turb_src_jac[sz0 + nz]);
+      out[NS + 5] = static_cast<double>(dq0[NS + 5]) + dt * tot[5 + NS] / (diag - dt * B.turb_src_jac[nz]);
+      out[NS + 6] = static_cast<double>(dq0[NS + 6]) + dt * tot[6 + NS] / (diag - dt * B.turb_src_jac[sz0 + nz]);
     } else {
-      out[NS + 5] = static_cast<double>(dq0[(NS + 5) * szd + nd]) + dt * tot[5 + NS] / diag;
-      out[NS + 6] = static_cast<double>(dq0[(NS + 6) * szd + nd]) + dt * tot[6 + NS] / diag;
+      out[NS + 5] = static_cast<double>(dq0[NS + 5]) + dt * tot[5 + NS] / diag;
+      out[NS + 6] = static_cast<double>(dq0[NS + 6]) + dt * tot[6 + NS] / diag;
     }
   }
   if (out_sel < 0) {
     OSTC_UNROLL for (int l = 0; l < NV; ++l) B.dq[l * szd + nd] = out[l];
   } else {
-    float *dqout = B.dqf[out_sel];
-    OSTC_UNROLL for (int l = 0; l < NV; ++l) dqout[l * szd + nd] = static_cast<float>(out[l]);
+    float d[NV];
+    OSTC_UNROLL for (int l = 0; l < NV; ++l) d[l] = static_cast<float>(out[l]);
+    B.terms32[out_sel * szd + nd] = pressure_term32<C>(B, n, nd, d);
+    store_increments32<C>(B.dqf[out_sel], szd, nd, d);
   }
 }
 

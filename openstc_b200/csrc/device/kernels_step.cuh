@@ -88,9 +88,6 @@ __global__ void __launch_bounds__(kCta, 4) k_source(const DevBlock *__restrict__
 #ifndef OSTC_FLUX_MIN_BLOCKS
 #define OSTC_FLUX_MIN_BLOCKS 4
 #endif
-#ifndef OSTC_SWEEP_MIN_BLOCKS
-#define OSTC_SWEEP_MIN_BLOCKS 4
-#endif
 
 // local_time_step, src/TimeAdvanceFunc.cuh:21-71: the spectral radii the
 // DPLUR stages use and the cell's local time step.
@@ -508,29 +505,118 @@ __global__ void __launch_bounds__(kCta) k_point_implicit(const DevBlock *__restr
   }
 }
 
-// compute_DQ_0, src/DPLURHPP.cuh:13-76.  Writes dq0; with EPI the factored
-// matrix replaces the Jacobian in chem_jac and the pivots go to lu_piv.
+// The terms of compute_jacobian_times_dq (src/DPLURHPP.cuh:78-125) that depend
+// on a cell's state and increments d but on no direction: the total enthalpy h
+// and the two pressure terms b2 and b3 - b4.  The kernel that writes d stores
+// them, so that a sweep does not sum over the species again for each of the six
+// neighbours that take them (54 quotients per cell).  hk(l): species enthalpy.
+// Explicit roundings where the compiler could contract in another way here than
+// in the reference's single expression.
+template <class C, class Hk>
+__device__ __forceinline__ void sweep_terms(const DevBlock &B, int64_t n, const double *d, Hk &&hk, double &h,
+                                            double &b2, double &b34) {
+  constexpr int NS = C::ns;
+  const int64_t sz = B.G.size;
+  const double u = ld(B.bv + sz + n), v = ld(B.bv + 2 * sz + n), w = ld(B.bv + 3 * sz + n);
+  const double vel = ld(B.vel + n);
+  const double e = __dmul_rn(0.5 * vel, vel);
+  double gamma = kDGammaAir, b3 = 0, b4 = 0;
+  h = 0;
+  if constexpr (C::mix != 0) {
+    const double t = ld(B.bv + 5 * sz + n);
+    gamma = ld(B.gamma + n);
+    OSTC_UNROLL for (int l = 0; l < NS; ++l) {
+      const double hl = hk(l);
+      b3 += kDR_u * t / cP.mw[l] * d[5 + l];
+      b4 += hl * d[5 + l];
+      h += ld(B.sv + l * sz + n) * hl;
+    }
+    b34 = __fma_rn(b3, gamma, -__dmul_rn(b4, gamma - 1));  // b3 - b4 as it contracts there
+    h += e;
+  } else {
+    b34 = 0;
+    h = gamma / (gamma - 1) * ld(B.bv + 4 * sz + n) / ld(B.bv + n) + e;
+  }
+  b2 = __fma_rn(e, d[0], -__dmul_rn(u, d[1]));
+  b2 = __dmul_rn(gamma - 1, __dadd_rn(__fma_rn(-w, d[3], __fma_rn(-v, d[2], b2)), d[4]));
+}
+
+// FP32-bulk path (kernels_mixed.cuh)
 template <class C>
-__global__ void __launch_bounds__(kCta) k_dq0(const DevBlock *__restrict__ blks, Tiles T) {
+__device__ __forceinline__ void sweep_terms32(const DevBlock &B, int64_t n, int64_t nd);
+template <class C>
+__device__ __forceinline__ void store_increments32(float4 *f, int64_t szd, int64_t nd, const float *d);
+
+// N doubles of this thread, `st` apart in global memory, into its slice of
+// shared memory (stride kCta) without passing through registers: all of them
+// are in flight at once, whatever registers the kernel has left.
+template <int N>
+__device__ __forceinline__ void copy_slice_async(double *slice, const double *src, int64_t st) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(slice));
+  OSTC_UNROLL for (int q = 0; q < N; ++q)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + q * kCta * 8), "l"(src + q * st) : "memory");
+}
+__device__ __forceinline__ void copy_slice_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Factors diag I - dt J (J in lhs, stride kCta), solves for rhs and stores the
+// factors and pivots.
+template <int N>
+__device__ __forceinline__ void dq0_epi(const DevBlock &B, int64_t nz, int64_t sz0, double dt, double diag, double *lhs,
+                                        double *rhs) {
+  OSTC_UNROLL for (int m = 0; m < N; ++m)
+    OSTC_UNROLL for (int q = 0; q < N; ++q) {
+      double &a = lhs[(m * N + q) * kCta];
+      a = (m == q) ? diag - dt * a : -dt * a;
+    }
+  int piv[N];
+  lu_factor<N, kCta>(lhs, piv);
+  lu_solve<N, kCta>(lhs, piv, rhs);
+  OSTC_UNROLL for (int q = 0; q < N * N; ++q) B.chem_jac[q * sz0 + nz] = lhs[q * kCta];
+  OSTC_UNROLL for (int q = 0; q < N; ++q) B.lu_piv[q * sz0 + nz] = static_cast<unsigned char>(piv[q]);
+}
+
+// The same through registers, R values in flight at a time (the loads are
+// volatile so that they stay together: left to the compiler they alternate with
+// the stores to shared memory, one memory latency each).
+template <int N, int R>
+__device__ __forceinline__ void copy_slice_batched(double *slice, const double *src, int64_t st) {
+  static_assert(N % R == 0);
+  OSTC_UNROLL for (int q = 0; q < N; q += R) {
+    double v[R];
+    OSTC_UNROLL for (int e = 0; e < R; ++e)
+      asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[e]) : "l"(src + (q + e) * st) : "memory");
+    OSTC_UNROLL for (int e = 0; e < R; ++e) slice[(q + e) * kCta] = v[e];
+  }
+}
+
+// compute_DQ_0, src/DPLURHPP.cuh:13-76.  Writes dq0; with EPI the factored
+// matrix replaces the Jacobian in chem_jac and the pivots go to lu_piv.  The
+// matrix of a thread lives in its slice of shared memory: N x N x 128 doubles, so
+// that two CTAs of 9 x 9 or three of 8 x 8 fit an SM.
+template <class C>
+__global__ void __launch_bounds__(kCta, C::mixed ? 3 : 2) k_dq0(const DevBlock *__restrict__ blks, Tiles T) {
   constexpr int NS = C::ns, NV = C::nv;
   int b, i, j, k;
   if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
   const DevBlock &B = blks[b];
   const int64_t nd = B.D.at(i, j, k), nz = B.Z.at(i, j, k), szd = B.D.size, sz0 = B.Z.size;
+  [[maybe_unused]] double *lhs = nullptr;
+  if constexpr (C::mix == 2) {
+    extern __shared__ double sdq[];
+    lhs = sdq + threadIdx.x + kTX * (threadIdx.y + kTY * threadIdx.z);
+    if (cP.chem_src_method == 1 && !(B.chem_quiet && B.chem_quiet[nz])) {
+      if (!C::mixed)
+        copy_slice_batched<NS * NS, 3 * NS>(lhs, B.chem_jac + nz, sz0);
+      else if (cP.na == NS - 1)
+        copy_slice_async<(NS - 1) * (NS - 1)>(lhs, B.chem_jac + nz, sz0);
+      else
+        copy_slice_async<NS * NS>(lhs, B.chem_jac + nz, sz0);
+    }
+  }
   const double dt = B.dt_local[nz];
   const double diag = 1 + dt * (B.inv_spec[nd] + B.inv_spec[szd + nd] + B.inv_spec[2 * szd + nd]);
   double dq[NV];  // loaded before the first store, which would hold the loads back
   OSTC_UNROLL for (int l = 0; l < NV; ++l) dq[l] = B.dq[l * szd + nd];
-  if constexpr (C::mix != 0) {
-    // T is fixed during the sweeps: evaluate the species enthalpies once
-    double hk[NS];
-    enthalpy<NS>(B.bv[5 * B.G.size + B.G.at(i, j, k)], hk);
-    if constexpr (C::mixed) {
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) B.h_spec32[l * szd + nd] = static_cast<float>(hk[l]);
-    } else {
-      OSTC_UNROLL for (int l = 0; l < NS; ++l) B.h_spec[l * szd + nd] = hk[l];
-    }
-  }
   if constexpr (C::mix != 2) {
     OSTC_UNROLL for (int l = 0; l < 5 + NS; ++l) dq[l] /= diag;
   } else {
@@ -540,37 +626,16 @@ __global__ void __launch_bounds__(kCta) k_dq0(const DevBlock *__restrict__ blks,
       // no chemistry Jacobian: the factorisation of diag I is diag I, and
       // its solve divides by diag (bit for bit)
       OSTC_UNROLL for (int l = 0; l < NS; ++l) dq[5 + l] /= diag;
-    } else if (method == 1 && C::mixed && cP.na == NS - 1) {
-      // FP32-bulk path: the leading (NS-1) x (NS-1) block, the last species
-      // with its single pivot diag (what the full factorisation gives it)
-      extern __shared__ double sdq[];
-      double *lhs = sdq + threadIdx.x + kTX * (threadIdx.y + kTY * threadIdx.z);
-      constexpr int NA = NS > 1 ? NS - 1 : 1;
-      int piv[NA];
-      OSTC_UNROLL for (int m = 0; m < NA; ++m)
-        OSTC_UNROLL for (int q = 0; q < NA; ++q) {
-          const double J = B.chem_jac[(m * NA + q) * sz0 + nz];
-          lhs[(m * NA + q) * kCta] = (m == q) ? diag - dt * J : -dt * J;
-        }
-      lu_factor<NA, kCta>(lhs, piv);
-      lu_solve<NA, kCta>(lhs, piv, dq + 5);
-      OSTC_UNROLL for (int l = NA; l < NS; ++l) dq[5 + l] /= diag;
-      OSTC_UNROLL for (int q = 0; q < NA * NA; ++q) B.chem_jac[q * sz0 + nz] = lhs[q * kCta];
-      OSTC_UNROLL for (int q = 0; q < NA; ++q) B.lu_piv[q * sz0 + nz] = static_cast<unsigned char>(piv[q]);
     } else if (method == 1) {
-      // the matrix lives in this thread's slice of shared memory (stride kCta)
-      extern __shared__ double sdq[];
-      double *lhs = sdq + threadIdx.x + kTX * (threadIdx.y + kTY * threadIdx.z);
-      int piv[NS];
-      OSTC_UNROLL for (int m = 0; m < NS; ++m)
-        OSTC_UNROLL for (int q = 0; q < NS; ++q) {
-          const double J = B.chem_jac[(m * NS + q) * sz0 + nz];
-          lhs[(m * NS + q) * kCta] = (m == q) ? diag - dt * J : -dt * J;
-        }
-      lu_factor<NS, kCta>(lhs, piv);
-      lu_solve<NS, kCta>(lhs, piv, dq + 5);
-      OSTC_UNROLL for (int q = 0; q < NS * NS; ++q) B.chem_jac[q * sz0 + nz] = lhs[q * kCta];
-      OSTC_UNROLL for (int q = 0; q < NS; ++q) B.lu_piv[q * sz0 + nz] = static_cast<unsigned char>(piv[q]);
+      if constexpr (C::mixed) copy_slice_wait();
+      if (C::mixed && cP.na == NS - 1) {
+        // FP32-bulk path: the leading (NS-1) x (NS-1) block, the last species
+        // with its single pivot diag (what the full factorisation gives it)
+        dq0_epi<(NS > 1 ? NS - 1 : 1)>(B, nz, sz0, dt, diag, lhs, dq + 5);
+        dq[5 + NS - 1] /= diag;
+      } else {
+        dq0_epi<NS>(B, nz, sz0, dt, diag, lhs, dq + 5);
+      }
     } else if (method == 2) {
       OSTC_UNROLL for (int l = 0; l < NS; ++l) dq[5 + l] /= diag - dt * B.chem_jac[l * sz0 + nz];
     } else {
@@ -587,7 +652,9 @@ __global__ void __launch_bounds__(kCta) k_dq0(const DevBlock *__restrict__ blks,
     }
   }
   if constexpr (C::mixed) {
-    OSTC_UNROLL for (int l = 0; l < NV; ++l) B.dqf[0][l * szd + nd] = static_cast<float>(dq[l]);
+    float d[NV];
+    OSTC_UNROLL for (int l = 0; l < NV; ++l) d[l] = static_cast<float>(dq[l]);
+    store_increments32<C>(B.dqf[0], szd, nd, d);
     if (cP.dplur_inner_step == 0)
       OSTC_UNROLL for (int l = 0; l < NV; ++l) B.dq0[l * szd + nd] = dq[l];
   } else {
@@ -595,48 +662,59 @@ __global__ void __launch_bounds__(kCta) k_dq0(const DevBlock *__restrict__ blks,
   }
 }
 
+// The species enthalpies, which T fixes for the sweeps, and the direction-
+// independent terms of dq0.  A kernel of its own: the factorisation of k_dq0
+// leaves room for 8 warps per SM, at which these sums took 5 ms of a 384 x 192 x
+// 64 step.
+template <class C>
+__global__ void __launch_bounds__(kCta) k_sweep_terms(const DevBlock *__restrict__ blks, Tiles T) {
+  constexpr int NS = C::ns, NV = C::nv;
+  int b, i, j, k;
+  if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
+  const DevBlock &B = blks[b];
+  const int64_t n = B.G.at(i, j, k), nd = B.D.at(i, j, k), szd = B.D.size;
+  if constexpr (C::mixed) {
+    sweep_terms32<C>(B, n, nd);
+  } else {
+    double d[NV], hk[NS > 0 ? NS : 1];
+    OSTC_UNROLL for (int l = 0; l < NV; ++l) d[l] = ld(B.dq0 + l * szd + nd);
+    if constexpr (C::mix != 0) enthalpy<NS>(ld(B.bv + 5 * B.G.size + n), hk);
+    double h, b2, b34;
+    sweep_terms<C>(B, n, d, [&](int l) { return hk[l]; }, h, b2, b34);
+    if constexpr (C::mix != 0) OSTC_UNROLL for (int l = 0; l < NS; ++l) B.h_spec[l * szd + nd] = hk[l];
+    B.terms[nd] = h;
+    B.terms[3 * szd + nd] = b2;
+    B.terms[4 * szd + nd] = b34;
+  }
+}
+
 // compute_jacobian_times_dq, src/DPLURHPP.cuh:78-125, accumulated into tot
 // with weight +-0.5 (sign < 0 subtracts), for the neighbour n along the
-// run-time direction dir.  The species enthalpies come from h_spec (k_dq0).
+// run-time direction dir; its direction-independent terms come from
+// sweep_terms (buffer `in` of the increments).
 template <class C>
-__device__ __forceinline__ void add_jac_dq(const DevBlock &B, const double *__restrict__ dqin, int64_t n,
+__device__ __forceinline__ void add_jac_dq(const DevBlock &B, const double *__restrict__ dqin, int in, int64_t n,
                                            int64_t nd, int dir, double pm_sr, bool subtract, double *tot) {
-  constexpr int NS = C::ns, NV = C::nv;
+  constexpr int NV = C::nv;
   const int64_t sz = B.G.size, szd = B.D.size;
   const double *mr = B.metric + 3 * dir * sz;
   const double xi_x = ld(mr + n), xi_y = ld(mr + sz + n), xi_z = ld(mr + 2 * sz + n);
   const double u = ld(B.bv + sz + n), v = ld(B.bv + 2 * sz + n), w = ld(B.bv + 3 * sz + n);
   const double U = xi_x * u + xi_y * v + xi_z * w;
   const double lmd1 = U + pm_sr;
-  const double vel = ld(B.vel + n);
-  const double e = 0.5 * vel * vel;
-  double gamma = kDGammaAir, b3 = 0, b4 = 0, h = 0;
   double d[NV];
   OSTC_UNROLL for (int l = 0; l < NV; ++l) d[l] = ld(dqin + l * szd + nd);
-  if constexpr (C::mix != 0) {
-    double hk[NS];
-    const double t = ld(B.bv + 5 * sz + n);
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) hk[l] = ld(B.h_spec + l * szd + nd);
-    gamma = ld(B.gamma + n);
-    OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-      b3 += kDR_u * t / cP.mw[l] * d[5 + l];
-      b4 += hk[l] * d[5 + l];
-      h += ld(B.sv + l * sz + n) * hk[l];
-    }
-    b3 *= gamma;
-    b4 *= gamma - 1;
-    h += e;
-  } else {
-    h = gamma / (gamma - 1) * ld(B.bv + 4 * sz + n) / ld(B.bv + n) + e;
-  }
+  const double h = ld(B.terms + nd), b2 = ld(B.terms + (1 + 2 * in) * szd + nd),
+               b34 = ld(B.terms + (2 + 2 * in) * szd + nd);
   const double b1 = xi_x * d[1] + xi_y * d[2] + xi_z * d[3] - U * d[0];
-  const double b2 = (gamma - 1) * (e * d[0] - u * d[1] - v * d[2] - w * d[3] + d[4]);
   double o[NV];
   o[0] = b1 + lmd1 * d[0];
-  o[1] = u * b1 + xi_x * b2 + lmd1 * d[1] + xi_x * (b3 - b4);
-  o[2] = v * b1 + xi_y * b2 + lmd1 * d[2] + xi_y * (b3 - b4);
-  o[3] = w * b1 + xi_z * b2 + lmd1 * d[3] + xi_z * (b3 - b4);
-  o[4] = h * b1 + U * b2 + lmd1 * d[4] + U * (b3 - b4);
+  // the roundings of u b1 + xi_x b2 + lmd1 d + xi_x (b3 - b4) as that expression
+  // contracts where b2, b3 and b4 are computed beside it
+  o[1] = __fma_rn(xi_x, b34, __fma_rn(lmd1, d[1], __fma_rn(u, b1, __dmul_rn(xi_x, b2))));
+  o[2] = __fma_rn(xi_y, b34, __fma_rn(lmd1, d[2], __fma_rn(v, b1, __dmul_rn(xi_y, b2))));
+  o[3] = __fma_rn(xi_z, b34, __fma_rn(lmd1, d[3], __fma_rn(w, b1, __dmul_rn(xi_z, b2))));
+  o[4] = __fma_rn(U, b34, __fma_rn(lmd1, d[4], __fma_rn(h, b1, __dmul_rn(U, b2))));
   OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) o[5 + l] = lmd1 * d[5 + l] + ld(B.sv + l * sz + n) * b1;
   if (subtract) {
     OSTC_UNROLL for (int l = 0; l < NV; ++l) tot[l] -= 0.5 * o[l];
@@ -648,7 +726,8 @@ __device__ __forceinline__ void add_jac_dq(const DevBlock &B, const double *__re
 // DPLUR_inner_iteration, src/DPLURHPP.cuh:127-249: dqout = dq0 + dt*sum/diag
 // with the neighbours' A(+-)*dqin; the point-implicit blocks reuse the LU.
 template <class C>
-__global__ void __launch_bounds__(kCta, OSTC_SWEEP_MIN_BLOCKS) k_sweep(const DevBlock *__restrict__ blks, Tiles T, int in_sel, int out_sel) {
+__global__ void __launch_bounds__(kCta, 4) k_sweep(const DevBlock *__restrict__ blks, Tiles T,
+                                                                       int in_sel, int out_sel, bool last) {
   constexpr int NS = C::ns, NV = C::nv;
   int b, i, j, k;
   if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
@@ -673,7 +752,7 @@ __global__ void __launch_bounds__(kCta, OSTC_SWEEP_MIN_BLOCKS) k_sweep(const Dev
     const int64_t gs = d == 0 ? 1 : (d == 1 ? sx : sxy), ds = d == 0 ? 1 : (d == 1 ? dsx : dsxy);
     const int64_t on = plus ? n + gs : n - gs, od = plus ? nd + ds : nd - ds;
     const double sr = isr[d * szd + od];
-    add_jac_dq<C>(B, dqin, on, od, d, plus ? -sr : sr, plus, tot);
+    add_jac_dq<C>(B, dqin, in_sel, on, od, d, plus ? -sr : sr, plus, tot);
   }
   const double dt = B.dt_local[nz];
   const double diag = 1 + dt * (isr[nd] + isr[szd + nd] + isr[2 * szd + nd]);
@@ -708,6 +787,12 @@ __global__ void __launch_bounds__(kCta, OSTC_SWEEP_MIN_BLOCKS) k_sweep(const Dev
       out[NS + 5] = B.dq0[(NS + 5) * szd + nd] + dt * tot[5 + NS] / diag;
       out[NS + 6] = B.dq0[(NS + 6) * szd + nd] + dt * tot[6 + NS] / diag;
     }
+  }
+  if (!last) {
+    double h, b2, b34;
+    sweep_terms<C>(B, n, out, [&](int l) { return ld(B.h_spec + l * szd + nd); }, h, b2, b34);
+    B.terms[(1 + 2 * out_sel) * szd + nd] = b2;
+    B.terms[(2 + 2 * out_sel) * szd + nd] = b34;
   }
   OSTC_UNROLL for (int l = 0; l < NV; ++l) dqout[l * szd + nd] = out[l];
 }
@@ -1279,7 +1364,7 @@ __global__ void k_inner(const DevBlock *__restrict__ blks, const DevInner *__res
 // of k_inner).  set: 0 mu_t and lambda_t, 1 |V|, 2 the inviscid spectral
 // radii, 3 the DPLUR increments of buffer dq_sel (0 dq, 1 dq0, 2 dqk), 4 the
 // species enthalpies of the sweeps.
-enum HaloSet { kHaloTurb = 0, kHaloVel = 1, kHaloSpec = 2, kHaloDq = 3, kHaloHspec = 4 };
+enum HaloSet { kHaloTurb = 0, kHaloVel = 1, kHaloSpec = 2, kHaloDq = 3, kHaloEnthalpy = 4 };
 
 template <class C>
 __global__ void k_halo(const DevBlock *__restrict__ blks, const DevInner *__restrict__ faces, int fi, int set,
@@ -1317,9 +1402,9 @@ __global__ void k_halo(const DevBlock *__restrict__ blks, const DevInner *__rest
     double *dst = dq_sel == 0 ? B.dq : (dq_sel == 1 ? B.dq0 : B.dqk);
     const double *src = dq_sel == 0 ? Tb.dq : (dq_sel == 1 ? Tb.dq0 : Tb.dqk);
     OSTC_UNROLL for (int l = 0; l < C::nv; ++l) dst[l * sz + n] = src[l * tsz + tn];
-  } else if (set == kHaloHspec) {
-    if constexpr (C::ns > 0)
-      OSTC_UNROLL for (int l = 0; l < C::ns; ++l) B.h_spec[l * sz + n] = Tb.h_spec[l * tsz + tn];
+    for (int l = 1 + 2 * dq_sel; l < 3 + 2 * dq_sel; ++l) B.terms[l * sz + n] = Tb.terms[l * tsz + tn];
+  } else if (set == kHaloEnthalpy) {
+    B.terms[n] = Tb.terms[tn];
   }
 }
 
