@@ -193,7 +193,7 @@ __device__ __forceinline__ void chemistry(double density, double t, const double
   auto rate2 = [&](int r) { return FAST ? arrhenius_exp(cP.A2[r], cP.lnA2[r], cP.b2[r], cP.Ea2[r], ln_t, t_inv)
                                         : arrhenius(t, cP.A2[r], cP.b2[r], cP.Ea2[r]); };
   double c[NS];
-  OSTC_UNROLL for (int l = 0; l < NS; ++l) c[l] = density * Y[l] / cP.mw[l] * 1e-3;
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) c[l] = div_mw(density * Y[l], l) * 1e-3;
   double g[NS];
   if constexpr (FAST)
     gibbs_rt_fast<NS>(t, ln_t, t_inv, g);
@@ -315,7 +315,7 @@ __device__ __forceinline__ void chemistry_fixed(double density, double t, const 
   auto rate2 = [&](int r) { return FAST ? arrhenius_exp(cP.A2[r], cP.lnA2[r], cP.b2[r], cP.Ea2[r], ln_t, t_inv)
                                         : arrhenius(t, cP.A2[r], cP.b2[r], cP.Ea2[r]); };
   double c[NS];
-  OSTC_UNROLL for (int l = 0; l < NS; ++l) c[l] = __dmul_rn(density * Y[l] / cP.mw[l], 1e-3);
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) c[l] = __dmul_rn(div_mw(density * Y[l], l), 1e-3);
   double g[NS];
   if constexpr (FAST)
     gibbs_rt_fast<NS>(t, ln_t, t_inv, g);
@@ -527,8 +527,8 @@ __device__ __forceinline__ void inviscid_face(const DevBlock &B, int64_t n, int 
     double er = 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]);
     double mwl = 0, mwr = 0;
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-      mwl += pl[5 + l] / cP.mw[l];
-      mwr += pr[5 + l] / cP.mw[l];
+      mwl += div_mw(pl[5 + l], l);
+      mwr += div_mw(pr[5 + l], l);
     }
     const double tl = pl[4] / (pl[0] * kDR_u * mwl);
     const double tr = pr[4] / (pr[0] * kDR_u * mwr);
@@ -666,9 +666,9 @@ __device__ __forceinline__ void viscous_face(const DevBlock &B, int64_t n, int d
   double mut = 0;
   if constexpr (C::turb) mut = 0.5 * (ld(B.mut + n) + ld(B.mut + n1));
   const double viscosity = mul + mut;
-  double tau_xx = viscosity * (4 * u_x - 2 * v_y - 2 * w_z) / 3.0;
-  double tau_yy = viscosity * (4 * v_y - 2 * u_x - 2 * w_z) / 3.0;
-  double tau_zz = viscosity * (4 * w_z - 2 * u_x - 2 * v_y) / 3.0;
+  double tau_xx = div_3(viscosity * (4 * u_x - 2 * v_y - 2 * w_z));
+  double tau_yy = div_3(viscosity * (4 * v_y - 2 * u_x - 2 * w_z));
+  double tau_zz = div_3(viscosity * (4 * w_z - 2 * u_x - 2 * v_y));
   const double tau_xy = viscosity * (u_y + v_x);
   const double tau_xz = viscosity * (u_z + w_x);
   const double tau_yz = viscosity * (v_z + w_y);

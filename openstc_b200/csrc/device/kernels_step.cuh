@@ -527,7 +527,7 @@ __device__ __forceinline__ void sweep_terms(const DevBlock &B, int64_t n, const 
     gamma = ld(B.gamma + n);
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
       const double hl = hk(l);
-      b3 += kDR_u * t / cP.mw[l] * d[5 + l];
+      b3 += div_mw(kDR_u * t, l) * d[5 + l];
       b4 += hl * d[5 + l];
       h += ld(B.sv + l * sz + n) * hl;
     }
@@ -802,7 +802,7 @@ __global__ void __launch_bounds__(kCta, 4) k_sweep(const DevBlock *__restrict__ 
 template <int NS>
 __device__ __forceinline__ void newton_temperature(const double *Y, double rho, double e, double &t, double &p) {
   double mw = 0;
-  OSTC_UNROLL for (int l = 0; l < NS; ++l) mw += Y[l] / cP.mw[l];
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) mw += div_mw(Y[l], l);
   mw = 1 / mw;
   const double gas_const = kDR_u / mw;
   double err = 1;
@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blk
     double mw = 0, cp_tot = 0, cv = 0;
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
       Y[l] = B.sv[l * sz + n];
-      mw += Y[l] / cP.mw[l];
+      mw += div_mw(Y[l], l);
       cp_tot += Y[l] * cp[l];
       cv += Y[l] * (cp[l] - cP.ru_mw[l]);
     }
@@ -1063,7 +1063,7 @@ __global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blk
       const double vt = wilke_sum<NS>(vis, X, m);
       const double cond_temp = 1.065 * vt - 0.065 * X[m];
       viscosity += vis[m] * X[m] / vt;
-      const double lambda = vis[m] * (cp[m] + 1.25 * kDR_u / cP.mw[m]);
+      const double lambda = vis[m] * (cp[m] + div_mw(1.25 * kDR_u, m));
       conductivity += lambda * X[m] / cond_temp;
     }
     B.mul[n] = viscosity;
@@ -1528,7 +1528,7 @@ __global__ void __launch_bounds__(kCta) k_init_mut(const DevBlock *__restrict__ 
     double mw = 0, Y[NS];
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
       Y[l] = B.sv[l * sz + n];
-      mw += Y[l] / cP.mw[l];
+      mw += div_mw(Y[l], l);
     }
     mw = 1 / mw;
     mul = mixture_viscosity<NS>(t, mw, Y);

@@ -37,6 +37,22 @@ struct Cfg {
 
 __device__ __forceinline__ double ld(const double *p) { return __ldg(p); }
 
+// x / y for a divisor known in advance, with 1 / y = zh + zl: two operations
+// instead of a division (N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in
+// advance", IEEE Trans. Computers 53, 2004).  The quotient is the correctly
+// rounded one unless x / y lies within about 2^-100 of the middle between two
+// doubles (x neither infinite nor so small that x zl underflows).  The FP64 path
+// divides by W_k and by 3 some 150 times per cell and step.
+__device__ __forceinline__ double div_by(double x, double zh, double zl) {
+  return __fma_rn(x, zh, __dmul_rn(x, zl));
+}
+__device__ __forceinline__ double div_mw(double x, int l) { return div_by(x, cP.mw_h[l], cP.mw_l[l]); }
+__device__ __forceinline__ double div_3(double x) {
+  constexpr double zh = 1.0 / 3.0, zl = 1.850371707708594e-17;  // 1 / 3 - zh
+  return div_by(x, zh, zl);
+}
+
 // ------------------------------------------------------------------ thermo
 // NASA-7 coefficient q of species i at temperature t (two ranges).
 __device__ __forceinline__ double nasa(int i, int q, bool lowrange) {
@@ -53,12 +69,12 @@ __device__ __forceinline__ void enthalpy(double t, double *h) {
       const double tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tt5 = tt4 * tt;
       const double c0 = cP.low[i * 7], c1 = cP.low[i * 7 + 1], c2 = cP.low[i * 7 + 2], c3 = cP.low[i * 7 + 3],
                    c4 = cP.low[i * 7 + 4], c5 = cP.low[i * 7 + 5];
-      h[i] = c0 * tt + 0.5 * c1 * tt2 + c2 * tt3 / 3 + 0.25 * c3 * tt4 + 0.2 * c4 * tt5 + c5;
+      h[i] = c0 * tt + 0.5 * c1 * tt2 + div_3(c2 * tt3) + 0.25 * c3 * tt4 + 0.2 * c4 * tt5 + c5;
       const double cp = c0 + c1 * tt + c2 * tt2 + c3 * tt3 + c4 * tt4;
       h[i] += cp * (t - tt);
     } else {
       const bool lo = t < cP.t_mid[i];
-      h[i] = nasa(i, 0, lo) * t + 0.5 * nasa(i, 1, lo) * t2 + nasa(i, 2, lo) * t3 / 3 + 0.25 * nasa(i, 3, lo) * t4 +
+      h[i] = nasa(i, 0, lo) * t + 0.5 * nasa(i, 1, lo) * t2 + div_3(nasa(i, 2, lo) * t3) + 0.25 * nasa(i, 3, lo) * t4 +
              0.2 * nasa(i, 4, lo) * t5 + nasa(i, 5, lo);
     }
     h[i] = __dmul_rn(h[i], cP.ru_mw[i]);
@@ -75,12 +91,12 @@ __device__ __forceinline__ void enthalpy_cp(double t, double *h, double *cp) {
       const double tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tt5 = tt4 * tt;
       const double c0 = cP.low[i * 7], c1 = cP.low[i * 7 + 1], c2 = cP.low[i * 7 + 2], c3 = cP.low[i * 7 + 3],
                    c4 = cP.low[i * 7 + 4], c5 = cP.low[i * 7 + 5];
-      h[i] = c0 * tt + 0.5 * c1 * tt2 + c2 * tt3 / 3 + 0.25 * c3 * tt4 + 0.2 * c4 * tt5 + c5;
+      h[i] = c0 * tt + 0.5 * c1 * tt2 + div_3(c2 * tt3) + 0.25 * c3 * tt4 + 0.2 * c4 * tt5 + c5;
       cp[i] = c0 + c1 * tt + c2 * tt2 + c3 * tt3 + c4 * tt4;
       h[i] += cp[i] * (t - tt);
     } else {
       const bool lo = t < cP.t_mid[i];
-      h[i] = nasa(i, 0, lo) * t + 0.5 * nasa(i, 1, lo) * t2 + nasa(i, 2, lo) * t3 / 3 + 0.25 * nasa(i, 3, lo) * t4 +
+      h[i] = nasa(i, 0, lo) * t + 0.5 * nasa(i, 1, lo) * t2 + div_3(nasa(i, 2, lo) * t3) + 0.25 * nasa(i, 3, lo) * t4 +
              0.2 * nasa(i, 4, lo) * t5 + nasa(i, 5, lo);
       cp[i] = nasa(i, 0, lo) + nasa(i, 1, lo) * t + nasa(i, 2, lo) * t2 + nasa(i, 3, lo) * t3 + nasa(i, 4, lo) * t4;
     }
@@ -116,12 +132,12 @@ __device__ __forceinline__ void gibbs_rt(double t, double *g) {
       const double tt = cP.t_low[i];
       const double tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tt_inv = 1 / tt, log_tt = std::log(tt);
       const double *c = &cP.low[i * 7];
-      g[i] = c[0] * (1.0 - log_tt) - 0.5 * c[1] * tt - c[2] * tt2 / 6.0 - c[3] * tt3 / 12.0 - c[4] * tt4 * 0.05 +
+      g[i] = c[0] * (1.0 - log_tt) - 0.5 * c[1] * tt - 0.5 * div_3(c[2] * tt2) - 0.25 * div_3(c[3] * tt3) - c[4] * tt4 * 0.05 +
              c[5] * tt_inv - c[6];
     } else {
       const bool lo = t < cP.t_mid[i];
-      g[i] = nasa(i, 0, lo) * (1.0 - log_t) - 0.5 * nasa(i, 1, lo) * t - nasa(i, 2, lo) * t2 / 6.0 -
-             nasa(i, 3, lo) * t3 / 12.0 - nasa(i, 4, lo) * t4 * 0.05 + nasa(i, 5, lo) * t_inv - nasa(i, 6, lo);
+      g[i] = nasa(i, 0, lo) * (1.0 - log_t) - 0.5 * nasa(i, 1, lo) * t - 0.5 * div_3(nasa(i, 2, lo) * t2) -
+             0.25 * div_3(nasa(i, 3, lo) * t3) - nasa(i, 4, lo) * t4 * 0.05 + nasa(i, 5, lo) * t_inv - nasa(i, 6, lo);
     }
   }
 }
@@ -158,7 +174,7 @@ template <int NS>
 __device__ __forceinline__ void species_viscosity(double t, double mw_total, const double *Y, double *X, double *vis) {
   const double st = sqrt(t);
   OSTC_UNROLL for (int l = 0; l < NS; ++l) {
-    X[l] = Y[l] * mw_total / cP.mw[l];
+    X[l] = div_mw(Y[l] * mw_total, l);
     const double t_dl = t * cP.lj_inv[l];
     const double ci = 1.147 * std::pow(t_dl, -0.145) + std::pow(t_dl + 0.5, -2);
     vis[l] = cP.vis_coeff[l] * st / ci;

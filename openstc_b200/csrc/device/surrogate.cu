@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) k_label(const double *states, double *dy,
   double Y[NS], d[NS], mw_inv = 0;
   for (int k = 0; k < NS; ++k) {
     Y[k] = s[2 + k];
-    mw_inv += Y[k] / cP.mw[k];
+    mw_inv += div_mw(Y[k], k);
   }
   const double rho = s[1] / (kDR_u * s[0] * mw_inv);
   sur::epi_increment<NS, M>(s[0], rho, Y, s[11], sq + threadIdx.x, sq + cP.nr * blockDim.x + threadIdx.x, blockDim.x, d);

@@ -288,6 +288,8 @@ void Driver::build_dev_params() {
   for (int i = 0; i < ns; ++i) {
     p.mw[i] = spec.mw[i];
     p.ru_mw[i] = kRu / spec.mw[i];
+    p.mw_h[i] = 1.0 / spec.mw[i];
+    p.mw_l[i] = std::fma(-p.mw_h[i], spec.mw[i], 1.0) / spec.mw[i];
     p.t_low[i] = spec.t_low[i];
     p.t_mid[i] = spec.t_mid[i];
     for (int q = 0; q < 7; ++q) {

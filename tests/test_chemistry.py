@@ -147,3 +147,26 @@ def test_compile_time_mechanism_is_the_shipped_one(params):
     assert table("label[nr]") == list(params.label[:19])
     assert table("sf[nr][ns]") == list(params.stoi_f[:19 * 9])
     assert table("sb[nr][ns]") == list(params.stoi_b[:19 * 9])
+
+
+def test_division_by_known_divisors_is_correctly_rounded(params):
+    """div_by (physics.cuh) with 1 / y as the sum of two doubles gives x / y for
+    the divisors the FP64 path uses it for, the molecular weights and 3, over the
+    exponents its operands have: exact rational arithmetic stands in for the
+    fused multiply-add."""
+    import random
+    from fractions import Fraction as F
+
+    def fma(a, b, c):
+        return float(F(a) * F(b) + F(c))
+
+    rng = random.Random(7)
+    for y in [3.0] + list(params.mw[:9]):
+        zh = 1.0 / y
+        zl = fma(-zh, y, 1.0) / y
+        if y == 3.0:
+            assert zl == 1.850371707708594e-17  # the header's literal
+        for _ in range(500):
+            x = rng.choice([-1, 1]) * rng.uniform(1, 2) * 2.0 ** rng.randint(-200, 200)
+            assert fma(x, zh, x * zl) == x / y, (x, y)
+        assert fma(0.0, zh, 0.0 * zl) == 0.0
