@@ -71,6 +71,8 @@ class EngineT final : public Engine {
                  "copy inner");
     }
     make_all_tiles();
+    group_bcs();
+    group_inner();
     cuda_check(cudaMalloc(&d_partial_, sizeof(double) * 4 * tiles0_.begin[tiles0_.nblk]), "cudaMalloc partial");
     cuda_check(cudaMalloc(&d_res_, sizeof(double) * 4), "cudaMalloc res");
     cuda_check(cudaMalloc(&d_bad_, sizeof(unsigned int)), "cudaMalloc bad");
@@ -304,7 +306,7 @@ class EngineT final : public Engine {
         k_wall_distance<<<grid(tilesg_), block3(), 0, stream_>>>(d_blocks_, tilesg_, d_wall_,
                                                                 static_cast<int>(setup_.wall_points.size() / 3));
     }
-    if (p.dim == 2) launch_kcopy();
+    if (p.dim == 2) k_kcopy<C><<<plane_grid(), kCta, 0, stream_>>>(d_blocks_);
     launch_bcs();
     k_cv_from_bv<C><<<grid(tilesg_), block3(), 0, stream_>>>(d_blocks_, tilesg_);
     if constexpr (C::turb) k_init_mut<C><<<grid(tiles1_), block3(), 0, stream_>>>(d_blocks_, tiles1_);
@@ -411,25 +413,23 @@ class EngineT final : public Engine {
 
   int launches_per_step(bool store_last, bool residual) const override {
     const auto &p = setup_.params;
-    int n = 2;  // source, flux
-    if constexpr (C::mixed) n += (p.dim == 3 ? 2 : 1) + static_cast<int>(blocks_.size());  // pack + one pass per direction
+    int n = C::mix != 2 && !C::turb ? 1 : 2;  // (source,) flux
+    if constexpr (C::mixed) n += p.dim == 3 ? 3 : 2;  // pack + one pass per direction
     if (p.implicit_method == 1) {
       n += 1 + (p.dplur_inner_step > 0 ? 1 : 0) + p.dplur_inner_step;
     } else if ((C::mix == 2 && p.chem_src_method != 0) || (C::turb && p.turb_implicit == 1)) {
       n += 1;
     }
     n += 2;  // update, limiter
-    n += static_cast<int>(setup_.bcs.size());
-    n += static_cast<int>(setup_.inner.size());
-    if (p.dim == 2) n += static_cast<int>(blocks_.size());
-    n += 1;  // properties
+    n += static_cast<int>(bc_launches_.points.size() + inner_launches_.points.size());
+    if (p.dim == 2 && C::mixed) n += 1;
+    n += 1;  // properties (2-D FP64: with the plane copy)
     if (store_last) n += 1;
     if (residual) n += 2;
     if (sur_on_) n += (C::mixed ? 5 : 3) * static_cast<int>(blocks_.size());  // candidates, inference, judge (+ chemistry list)
-    if (setup_.exact_inner) {  // the halo copies of exact inner faces
-      int sets = 2;  // mu_t / lambda_t, |V|
-      if (p.implicit_method == 1) sets += 2 + p.dplur_inner_step;  // spectral radii, enthalpies, each sweep's input
-      n += sets * static_cast<int>(setup_.inner.size());
+    if (setup_.exact_inner && !setup_.inner.empty()) {  // the halo copies of exact inner faces
+      n += 2;  // mu_t / lambda_t, |V|
+      if (p.implicit_method == 1) n += 2 + p.dplur_inner_step;  // spectral radii, enthalpies, each sweep's input
     }
     return n;
   }
@@ -662,7 +662,9 @@ class EngineT final : public Engine {
 
   // How the flux kernels cut the grid.  Long columns or marches evaluate the
   // fewest faces, short ones keep the SMs of a small grid busy; the constants
-  // are from event times on one B200.  FP64 (reacting layer, in us):
+  // are from event times on one B200.  FP64 (reacting layer, in us; taken
+  // before the divisions by constants became products (div_by), which made a
+  // full grid 17 % faster: 160 x 96 x 64 is 2.7 ms now; the order is the same):
   //   24 x 16 x 8:    8 / 4 / 2 / 1 planes 652 / 344 / 190 / 112, rows 24
   //   45 x 37 x 21:                        707 / 381 / 225 / 240, rows 217
   //   96 x 64 x 32:                        909 / 872 / 724 / 768, rows 868
@@ -768,10 +770,12 @@ class EngineT final : public Engine {
     }
   }
 
-  void launch_flux() {
+  // fresh: no source stage ran, dq starts at zero (laminar air)
+  void launch_flux(bool fresh = false) {
     if constexpr (C::mixed) {
-      for (int b = 0; b < static_cast<int>(blocks_.size()); ++b)
-        k_pack32<C><<<pack_grid(b), 256, 0, stream_>>>(d_blocks_, b);
+      unsigned most = 0;
+      for (int b = 0; b < static_cast<int>(blocks_.size()); ++b) most = std::max(most, pack_grid(b));
+      k_pack32<C><<<dim3(most, static_cast<unsigned>(blocks_.size())), 256, 0, stream_>>>(d_blocks_);
       mark("pack32");
       switch (flux_variant_) {
         case 0: launch_flux_passes<kFluxVariant[0].min_blocks>(); break;
@@ -781,11 +785,11 @@ class EngineT final : public Engine {
       }
     } else if (flux_variant_ == 1) {
       // the per-cell form: each face evaluated by both of its cells, no barriers
-      k_flux<C><<<grid(tiles0_), block3(), flux_smem_, stream_>>>(d_blocks_, tiles0_);
+      k_flux<C><<<grid(tiles0_), block3(), flux_smem_, stream_>>>(d_blocks_, tiles0_, fresh);
     } else if (row_warps_ > 0) {
-      k_flux_row<C><<<grid(col_tiles_), dim3(32, row_warps_), 0, stream_>>>(d_blocks_, col_tiles_);
+      k_flux_row<C><<<grid(col_tiles_), dim3(32, row_warps_), 0, stream_>>>(d_blocks_, col_tiles_, fresh);
     } else {
-      k_flux_col<C><<<grid(col_tiles_), kFluxThreads, col_smem_, stream_>>>(d_blocks_, col_tiles_, col_kc_);
+      k_flux_col<C><<<grid(col_tiles_), kFluxThreads, col_smem_, stream_>>>(d_blocks_, col_tiles_, col_kc_, fresh);
     }
   }
 
@@ -803,9 +807,9 @@ class EngineT final : public Engine {
 
   void launch_props() {
     if constexpr (C::mixed)
-      k_props_mx<C><<<grid(tiles1_), block3(), 0, stream_>>>(d_blocks_, tiles1_);
+      k_props_mx<C><<<grid(tiles1_), block3(), 0, stream_>>>(d_blocks_, tiles1_, d_bad_);
     else
-      k_props<C><<<grid(tiles1_), block3(), 0, stream_>>>(d_blocks_, tiles1_);
+      k_props<C><<<grid(tiles1_), block3(), 0, stream_>>>(d_blocks_, tiles1_, d_bad_);
   }
 
   // the surrogate marks chemically quiet cells before the source term
@@ -836,10 +840,13 @@ class EngineT final : public Engine {
 
   void launch_residual() {
     if (sur_on_) launch_classify();
-    launch_source();
-    mark("source");
+    constexpr bool no_source = C::mix != 2 && !C::turb;  // the source stage would only zero dq
+    if constexpr (!no_source) {
+      launch_source();
+      mark("source");
+    }
     launch_halo(kHaloTurb);
-    launch_flux();
+    launch_flux(no_source);
     if constexpr (!C::mixed) mark("flux");
     launch_halo(kHaloSpec);
   }
@@ -980,32 +987,129 @@ class EngineT final : public Engine {
   }
 
   void launch_update() {
-    cuda_check(cudaMemsetAsync(d_bad_, 0, sizeof(unsigned int), stream_), "memset bad");
-    mark("memset");
     k_update<C><<<grid(tiles0_), block3(), 0, stream_>>>(d_blocks_, tiles0_, final_dq_, d_bad_);
     mark("update");
     k_limit<C><<<grid(tiles0_), block3(), 0, stream_>>>(d_blocks_, tiles0_, d_bad_);
     mark("limit_flow");
   }
 
+  // A box of points that a face kernel reads or writes in a block.
+  struct Touch {
+    int block, lo[3], hi[3];
+    bool meets(const Touch &o) const {
+      if (block != o.block) return false;
+      for (int d = 0; d < 3; ++d)
+        if (hi[d] < o.lo[d] || o.hi[d] < lo[d]) return false;
+      return true;
+    }
+  };
+
+  // Groups faces into launches: a face goes into the launch after the last
+  // earlier face that touches one of its points, so that every pair of faces
+  // whose order could matter keeps it.  order: face indices launch by launch
+  // (device), first[l]: the launch's first entry, points[l]: its largest face.
+  struct FaceLaunches {
+    int *order = nullptr;
+    std::vector<int> first, points;
+  };
+
+  FaceLaunches group_faces(const std::vector<std::vector<Touch>> &touch, const std::vector<int> &points) {
+    const int n = static_cast<int>(touch.size());
+    std::vector<int> level(n, 0);
+    int levels = 0;
+    for (int q = 0; q < n; ++q) {
+      if (points[q] <= 0) continue;
+      for (int e = 0; e < q; ++e) {
+        if (points[e] <= 0) continue;
+        bool meet = false;
+        for (const Touch &x : touch[q])
+          for (const Touch &y : touch[e]) meet = meet || x.meets(y);
+        if (meet) level[q] = std::max(level[q], level[e] + 1);
+      }
+      levels = std::max(levels, level[q] + 1);
+    }
+    FaceLaunches g;
+    std::vector<int> order;
+    for (int l = 0; l < levels; ++l) {
+      g.first.push_back(static_cast<int>(order.size()));
+      g.points.push_back(0);
+      for (int q = 0; q < n; ++q)
+        if (points[q] > 0 && level[q] == l) {
+          order.push_back(q);
+          g.points[l] = std::max(g.points[l], points[q]);
+        }
+    }
+    g.first.push_back(static_cast<int>(order.size()));
+    if (!order.empty()) {
+      void *d = nullptr;
+      cuda_check(cudaMalloc(&d, sizeof(int) * order.size()), "cudaMalloc face order");
+      allocations_.push_back(d);
+      g.order = static_cast<int *>(d);
+      cuda_check(cudaMemcpyAsync(d, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, stream_),
+                 "copy face order");
+      cuda_check(cudaStreamSynchronize(stream_), "copy face order");
+    }
+    return g;
+  }
+
+  // k_bc touches ngg layers on both sides of its face
+  void group_bcs() {
+    std::vector<std::vector<Touch>> touch;
+    std::vector<int> points;
+    for (const HostBc &f : setup_.bcs) {
+      Touch t{f.block, {f.start[0], f.start[1], f.start[2]}, {f.end[0], f.end[1], f.end[2]}};
+      t.lo[f.face] -= setup_.ngg;
+      t.hi[f.face] += setup_.ngg;
+      touch.push_back({t});
+      points.push_back((f.end[0] - f.start[0] + 1) * (f.end[1] - f.start[1] + 1) * (f.end[2] - f.start[2] + 1));
+    }
+    bc_launches_ = group_faces(touch, points);
+  }
+
+  // k_inner touches its own points (plane and ghosts, with exact faces also the
+  // tangential ghost rows) and the points they map to in the other block
+  void group_inner() {
+    std::vector<std::vector<Touch>> touch;
+    std::vector<int> points;
+    const int tg = setup_.exact_inner ? setup_.ngg : 0;
+    for (const HostInner &f : setup_.inner) {
+      Touch own{f.block, {}, {}}, other{f.target_block, {}, {}};
+      int lo[3], hi[3], np = 1;  // range of d = loop_dir * n
+      for (int q = 0; q < 3; ++q) {
+        const int wide = q != f.face && f.n_point[q] > 1 ? tg : 0;
+        const int e0 = f.loop_dir[q] * -wide, e1 = f.loop_dir[q] * (f.n_point[q] - 1 + wide);
+        lo[q] = std::min(e0, e1);
+        hi[q] = std::max(e0, e1);
+        own.lo[q] = f.start[q] + lo[q];
+        own.hi[q] = f.start[q] + hi[q];
+        np *= f.n_point[q] + 2 * wide;
+      }
+      for (int q = 0; q < 3; ++q) {
+        const int e0 = f.tstart[q] + f.tloop_dir[q] * lo[f.src_tar[q]], e1 = f.tstart[q] + f.tloop_dir[q] * hi[f.src_tar[q]];
+        other.lo[q] = std::min(e0, e1);
+        other.hi[q] = std::max(e0, e1);
+      }
+      touch.push_back({own, other});
+      points.push_back(f.n_point[0] * f.n_point[1] * f.n_point[2] > 0 ? np : 0);
+    }
+    inner_launches_ = group_faces(touch, points);
+  }
+
   void launch_bcs() {
-    for (int q = 0; q < static_cast<int>(setup_.bcs.size()); ++q) {
-      const HostBc &f = setup_.bcs[q];
-      const int np = (f.end[0] - f.start[0] + 1) * (f.end[1] - f.start[1] + 1) * (f.end[2] - f.start[2] + 1);
-      if (np <= 0) continue;
-      k_bc<C><<<(np + 127) / 128, 128, 0, stream_>>>(d_blocks_, d_bcs_, q);
+    const FaceLaunches &g = bc_launches_;
+    for (size_t l = 0; l + 1 < g.first.size(); ++l) {
+      const dim3 grid((g.points[l] + 127) / 128, g.first[l + 1] - g.first[l]);
+      k_bc<C><<<grid, 128, 0, stream_>>>(d_blocks_, d_bcs_, g.order + g.first[l]);
       mark("boundary");
     }
   }
 
   void launch_inner() {
-    for (int q = 0; q < static_cast<int>(setup_.inner.size()); ++q) {
-      const HostInner &f = setup_.inner[q];
-      if (f.n_point[0] * f.n_point[1] * f.n_point[2] <= 0) continue;
-      const int tg = setup_.exact_inner ? setup_.ngg : 0;
-      int np = 1;
-      for (int d = 0; d < 3; ++d) np *= f.n_point[d] + (d != f.face && f.n_point[d] > 1 ? 2 * tg : 0);
-      k_inner<C><<<(np + 127) / 128, 128, 0, stream_>>>(d_blocks_, d_inner_, q, setup_.exact_inner, tg);
+    const FaceLaunches &g = inner_launches_;
+    const int tg = setup_.exact_inner ? setup_.ngg : 0;
+    for (size_t l = 0; l + 1 < g.first.size(); ++l) {
+      const dim3 grid((g.points[l] + 127) / 128, g.first[l + 1] - g.first[l]);
+      k_inner<C><<<grid, 128, 0, stream_>>>(d_blocks_, d_inner_, g.order + g.first[l], setup_.exact_inner, tg);
       mark("inner_face");
     }
     launch_halo(kHaloVel);
@@ -1017,13 +1121,12 @@ class EngineT final : public Engine {
     if (!setup_.exact_inner) return;
     // the spectral radii, increments and enthalpies have their ghost layer under DPLUR only
     if (set != kHaloTurb && set != kHaloVel && setup_.params.implicit_method != 1) return;
-    for (int q = 0; q < static_cast<int>(setup_.inner.size()); ++q) {
-      const HostInner &f = setup_.inner[q];
-      const int np = f.n_point[0] * f.n_point[1] * f.n_point[2];
-      if (np <= 0) continue;
-      k_halo<C><<<(np + 127) / 128, 128, 0, stream_>>>(d_blocks_, d_inner_, q, set, dq_sel);
-      mark("halo");
-    }
+    int np = 0;
+    for (const HostInner &f : setup_.inner) np = std::max(np, f.n_point[0] * f.n_point[1] * f.n_point[2]);
+    if (np <= 0) return;
+    k_halo<C><<<dim3((np + 127) / 128, static_cast<unsigned>(setup_.inner.size())), 128, 0, stream_>>>(d_blocks_, d_inner_,
+                                                                                                      set, dq_sel);
+    mark("halo");
   }
 
   // The bucket grid of the wall points for k_wall_distance_grid: method 2, or
@@ -1112,18 +1215,26 @@ class EngineT final : public Engine {
     }
   }
 
-  void launch_kcopy() {
-    for (int b = 0; b < static_cast<int>(blocks_.size()); ++b) {
-      const DevBlock &B = blocks_[b];
-      const int np = (B.mx + 2 * B.ngg) * (B.my + 2 * B.ngg);
-      k_kcopy<C><<<(np + 127) / 128, 128, 0, stream_>>>(d_blocks_, b);
-      mark("k_copy");
-    }
+  // one thread per column of a 2-D case, ghosts included, over every block
+  dim3 plane_grid() const {
+    int np = 0;
+    for (const auto &B : blocks_) np = std::max(np, (B.mx + 2 * B.ngg) * (B.my + 2 * B.ngg));
+    return dim3((np + kCta - 1) / kCta, static_cast<unsigned>(blocks_.size()));
   }
 
   void launch_exchange() {
     launch_inner();
-    if (setup_.params.dim == 2) launch_kcopy();
+    if constexpr (!C::mixed) {
+      if (setup_.params.dim == 2) {
+        k_plane_props<C><<<plane_grid(), kCta, 0, stream_>>>(d_blocks_, d_bad_);
+        mark("properties");
+        return;
+      }
+    }
+    if (setup_.params.dim == 2) {
+      k_kcopy<C><<<plane_grid(), kCta, 0, stream_>>>(d_blocks_);
+      mark("k_copy");
+    }
     launch_props();
     mark("properties");
   }
@@ -1219,6 +1330,7 @@ class EngineT final : public Engine {
   std::vector<int> order_;  // the blocks' schedule in every tile table (empty: block order)
   int flux_variant_ = 0;    // kFluxVariant entry of the FP32-bulk flux passes
   int march_[3] = {1, 1, 1};  // cells a thread of the y / z pass marches over
+  FaceLaunches bc_launches_, inner_launches_;
   int col_kc_ = kFluxKC;      // planes of a column (k_flux_col) ...
   int row_warps_ = 0;         // ... or, when positive, the warps of a row (k_flux_row)
   WallGrid wall_grid_{};    // the bucket grid of the wall points (start null: brute force)

@@ -705,11 +705,11 @@ __device__ __forceinline__ void face_g(const DevBlock &B, int64_t nl, int d, int
 
 // The FP32 copy of the operands of the direction passes, over every point of
 // layout G: the fields that change every step (after the source stage, which
-// writes mu_t and lambda_t) ...
+// writes mu_t and lambda_t; blockIdx.y: block) ...
 template <class C>
-__global__ void __launch_bounds__(256) k_pack32(const DevBlock *__restrict__ blks, int b) {
+__global__ void __launch_bounds__(256) k_pack32(const DevBlock *__restrict__ blks) {
   using Q = fp32::Quad;
-  const DevBlock &B = blks[b];
+  const DevBlock &B = blks[blockIdx.y];
   const int64_t sz = B.G.size;
   float4 *f = B.f32;
   for (int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; n < sz;
@@ -991,7 +991,9 @@ __global__ void __launch_bounds__(kCta, 4) k_sweep_mx(const DevBlock *__restrict
 
 // Thermodynamic and transport properties in FP32 (update_physical_properties).
 template <class C>
-__global__ void __launch_bounds__(kCta) k_props_mx(const DevBlock *__restrict__ blks, Tiles T) {
+__global__ void __launch_bounds__(kCta) k_props_mx(const DevBlock *__restrict__ blks, Tiles T,
+                                                   unsigned int *bad_count) {
+  if (blockIdx.x == 0 && threadIdx.x + threadIdx.y == 0) *bad_count = 0;
   constexpr int NS = C::ns;
   using fp32::ldf;
   int b, i, j, k;

@@ -130,9 +130,11 @@ __device__ __forceinline__ void local_time_step(const DevBlock &B, int i, int j,
 // ---------------------------------------------------------------- fluxes
 // Inviscid (AUSM+/MUSCL) then viscous (central) flux differences in the
 // reference's accumulation order, plus local_time_step
-// (src/TimeAdvanceFunc.cuh:21-71).
+// (src/TimeAdvanceFunc.cuh:21-71).  fresh: there is no source term (laminar
+// air), dq starts at zero.
 template <class C>
-__global__ void __launch_bounds__(kCta, OSTC_FLUX_MIN_BLOCKS) k_flux(const DevBlock *__restrict__ blks, Tiles T) {
+__global__ void __launch_bounds__(kCta, OSTC_FLUX_MIN_BLOCKS) k_flux(const DevBlock *__restrict__ blks, Tiles T,
+                                                                      bool fresh) {
   constexpr int NV = C::nv;
   extern __shared__ double sf[];
   int b, i, j, k;
@@ -144,7 +146,7 @@ __global__ void __launch_bounds__(kCta, OSTC_FLUX_MIN_BLOCKS) k_flux(const DevBl
   const int64_t sx = B.G.sx, sxy = B.G.sxy;
   const bool three_d = B.mz > 1;
   double dq[NV];
-  OSTC_UNROLL for (int l = 0; l < NV; ++l) dq[l] = B.dq[l * szd + nd];
+  OSTC_UNROLL for (int l = 0; l < NV; ++l) dq[l] = fresh ? 0.0 : B.dq[l * szd + nd];
   // Inviscid faces, then viscous faces, each direction as minus face (staged
   // in shared memory) then plus face: dq -= f(+) - f(-) for inviscid and
   // dq += f(+) - f(-) for viscous, the reference's accumulation order.  The
@@ -302,7 +304,7 @@ __device__ __forceinline__ void col_faces64(const DevBlock &B, int i0, int j0, i
 
 template <class C>
 __global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__restrict__ blks, Tiles T,
-                                                               int kc) {
+                                                               int kc, bool fresh) {
   constexpr int NV = C::nv;
   extern __shared__ double sm64[];
   int b, i0, j0, k0;
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__
     if (cell) {
       n = B.G.at(i, j, k);
       nd = B.D.at(i, j, k);
-      OSTC_UNROLL for (int l = 0; l < NV; ++l) dq[l] = B.dq[l * szd + nd];
+      OSTC_UNROLL for (int l = 0; l < NV; ++l) dq[l] = fresh ? 0.0 : B.dq[l * szd + nd];
     }
     col_faces64<C, 0>(B, i0, j0, k, k == k0, cell, sm64, dq);
     if (cP.viscous_order != 0) col_faces64<C, 1>(B, i0, j0, k, k == k0, cell, sm64, dq);
@@ -341,7 +343,7 @@ constexpr int kRowFaces = 6;
 
 template <class C>
 __global__ void __launch_bounds__(2 * kRowFaces * 32, C::mix == 0 ? 2 : 1)
-    k_flux_row(const DevBlock *__restrict__ blks, Tiles T) {
+    k_flux_row(const DevBlock *__restrict__ blks, Tiles T, bool fresh) {
   constexpr int NV = C::nv;
   __shared__ double sm[2 * kRowFaces * NV * 32];
   int b;
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(2 * kRowFaces * 32, C::mix == 0 ? 2 : 1)
   __syncthreads();
   if (!cell) return;
   for (int l = w; l < NV; l += blockDim.y) {
-    double dq = B.dq[l * szd + nd];
+    double dq = fresh ? 0.0 : B.dq[l * szd + nd];
     for (int f = 0; f < n_face; f += 2) dq -= sm[((f + 1) * NV + l) * 32 + lane] - sm[(f * NV + l) * 32 + lane];
     if (visc)
       for (int f = n_face; f < 2 * n_face; f += 2)
@@ -1029,17 +1031,24 @@ __global__ void __launch_bounds__(kCta) k_limit(const DevBlock *__restrict__ blk
 }
 
 // update_physical_properties + compute_transport_property,
-// src/FieldOperation.cuh:75-109, src/Transport.cu:40-84 (interior + one
-// ghost layer: launched with halo 1).
-template <class C>
-__global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blks, Tiles T) {
+// src/FieldOperation.cuh:75-109, src/Transport.cu:40-84, of point n (PLANES: and
+// the same values at the points above and below it, whose state is the same).
+template <class C, bool PLANES>
+__device__ __forceinline__ void point_properties(const DevBlock &B, int64_t n) {
   constexpr int NS = C::ns;
-  int b, i, j, k;
-  if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
-  const DevBlock &B = blks[b];
-  const int64_t n = B.G.at(i, j, k), sz = B.G.size;
+  const int64_t sz = B.G.size, sxy = B.G.sxy;
   const double t = B.bv[5 * sz + n];
-  const double speed = B.vel[n];  // read before the first store, which would hold it back
+  // every load before the first store, which would hold it back
+  double speed[3];
+  OSTC_UNROLL for (int q = 0; q < 3; ++q) speed[q] = PLANES || q == 1 ? B.vel[n + (q - 1) * sxy] : 0.0;
+  auto put = [&](double *x, double v) {
+    x[n] = v;
+    if constexpr (PLANES) x[n - sxy] = x[n + sxy] = v;
+  };
+  auto put_mach = [&](double a) {
+    OSTC_UNROLL for (int q = 0; q < 3; ++q)
+      if (PLANES || q == 1) B.mach[n + (q - 1) * sxy] = speed[q] / a;
+  };
   if constexpr (C::mix != 0) {
     double cp[NS], Y[NS];
     heat_capacity<NS>(t, cp);
@@ -1052,10 +1061,10 @@ __global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blk
     }
     mw = 1 / mw;
     const double gamma = cp_tot / cv;
-    B.cp[n] = cp_tot;
-    B.gamma[n] = gamma;
+    put(B.cp, cp_tot);
+    put(B.gamma, gamma);
     const double a = sqrt(gamma * kDR_u * t / mw);
-    B.acoustic[n] = a;
+    put(B.acoustic, a);
     double X[NS], vis[NS];
     species_viscosity<NS>(t, mw, Y, X, vis);
     double viscosity = 0, conductivity = 0;
@@ -1066,8 +1075,8 @@ __global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blk
       const double lambda = vis[m] * (cp[m] + div_mw(1.25 * kDR_u, m));
       conductivity += lambda * X[m] / cond_temp;
     }
-    B.mul[n] = viscosity;
-    B.cond[n] = conductivity;
+    put(B.mul, viscosity);
+    put(B.cond, conductivity);
     const double sc = cP.Sc;
     OSTC_UNROLL for (int l = 0; l < NS; ++l) {
       double d;
@@ -1076,19 +1085,68 @@ __global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blk
       } else {
         d = (1 - Y[l]) * viscosity / ((1 - X[l]) * sc);
       }
-      B.rho_d[l * sz + n] = d;
+      put(B.rho_d + l * sz, d);
     }
-    B.mach[n] = speed / a;
+    put_mach(a);
   } else {
     constexpr double c_temp = kDGammaAir * kDR_u / kDMwAir;
     constexpr double cp = kDGammaAir * kDR_u / kDMwAir / (kDGammaAir - 1);
     const double a = sqrt(c_temp * t);
-    B.acoustic[n] = a;
+    put(B.acoustic, a);
     const double mul = sutherland(t);
-    B.mul[n] = mul;
-    B.cond[n] = mul * cp / cP.Pr;
-    B.mach[n] = speed / a;
+    put(B.mul, mul);
+    put(B.cond, mul * cp / cP.Pr);
+    put_mach(a);
   }
+}
+
+// Interior + one ghost layer: launched with halo 1.  The properties' kernels
+// also clear the bad-cell counter for the next update (the limiter, which reads
+// it, has run before them).
+template <class C>
+__global__ void __launch_bounds__(kCta) k_props(const DevBlock *__restrict__ blks, Tiles T, unsigned int *bad_count) {
+  if (blockIdx.x == 0 && threadIdx.x + threadIdx.y == 0) *bad_count = 0;
+  int b, i, j, k;
+  if (!tile_cell<kTX, kTY, kTZ>(T, b, i, j, k, blks)) return;
+  point_properties<C, false>(blks[b], blks[b].G.at(i, j, k));
+}
+
+// The plane's values of column n0 of a 2-D case into its ghost planes
+// (eliminate_k_gradient, src/FieldOperation.cu:42-62).
+template <class C>
+__device__ __forceinline__ void copy_plane(const DevBlock &B, int64_t n0) {
+  const int64_t sz = B.G.size;
+  // the plane's values read once, before the stores
+  double pb[6], ps[C::nsc > 0 ? C::nsc : 1];
+  OSTC_UNROLL for (int l = 0; l < 6; ++l) pb[l] = B.bv[l * sz + n0];
+  OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) ps[l] = B.sv[l * sz + n0];
+  for (int k = 1; k <= B.ngg; ++k) {
+    const int64_t np = n0 + k * B.G.sxy, nm = n0 - k * B.G.sxy;
+    OSTC_UNROLL for (int l = 0; l < 6; ++l) {
+      B.bv[l * sz + np] = pb[l];
+      B.bv[l * sz + nm] = pb[l];
+    }
+    OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) {
+      B.sv[l * sz + np] = ps[l];
+      B.sv[l * sz + nm] = ps[l];
+    }
+  }
+}
+
+// 2-D cases: the plane copied into the ghost planes and, within one ghost
+// layer, its properties evaluated once for the three planes that k_props
+// would evaluate, in one launch (256 x 128 ramp: two launches of 8 us).
+// blockIdx.y: block.
+template <class C>
+__global__ void __launch_bounds__(kCta) k_plane_props(const DevBlock *__restrict__ blks, unsigned int *bad_count) {
+  if (blockIdx.x + blockIdx.y + threadIdx.x == 0) *bad_count = 0;
+  const DevBlock &B = blks[blockIdx.y];
+  const int g = B.ngg, ex = B.mx + 2 * g, t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ex * (B.my + 2 * g)) return;
+  const int i = t % ex - g, j = t / ex - g;
+  const int64_t n = B.G.at(i, j, 0);
+  copy_plane<C>(B, n);
+  if (i >= -1 && i <= B.mx && j >= -1 && j <= B.my) point_properties<C, true>(B, n);
 }
 
 // ---------------------------------------------------------------- boundaries
@@ -1140,11 +1198,12 @@ __device__ __forceinline__ void total_energy(const DevBlock &B, int64_t n) {
 // tell the arrays apart, so a load written after a store would wait for that
 // store, one memory round trip per variable.  The arithmetic is the
 // reference's, in its order.
+// blockIdx.y: entry of `faces`, faces that touch no common point.
 template <class C>
-__global__ void k_bc(const DevBlock *__restrict__ blks, const DevBc *__restrict__ bcs, int face) {
+__global__ void k_bc(const DevBlock *__restrict__ blks, const DevBc *__restrict__ bcs, const int *__restrict__ faces) {
   constexpr int NS = C::ns, NSC = C::nsc;
   constexpr int NS1 = NS > 0 ? NS : 1, NSC1 = NSC > 0 ? NSC : 1;
-  const DevBc &f = bcs[face];
+  const DevBc &f = bcs[faces[blockIdx.y]];
   const int e0 = f.end[0] - f.start[0] + 1, e1 = f.end[1] - f.start[1] + 1, e2 = f.end[2] - f.start[2] + 1;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e0 * e1 * e2) return;
@@ -1322,10 +1381,11 @@ struct DevInner {
 // exact: the shared plane is computed identically by both blocks and is not
 // re-averaged, and the ghost copy also covers the face's tangential ghost
 // rows (tg = ngg), which the viscous stencils read next to the face
+// blockIdx.y: entry of `list`, faces that touch no common point.
 template <class C>
-__global__ void k_inner(const DevBlock *__restrict__ blks, const DevInner *__restrict__ faces, int fi, bool exact,
-                        int tg) {
-  const DevInner &f = faces[fi];
+__global__ void k_inner(const DevBlock *__restrict__ blks, const DevInner *__restrict__ faces,
+                        const int *__restrict__ list, bool exact, int tg) {
+  const DevInner &f = faces[list[blockIdx.y]];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   int ext[3];
   for (int q = 0; q < 3; ++q) ext[q] = f.n_point[q] + (q != f.face && f.n_point[q] > 1 ? 2 * tg : 0);
@@ -1367,9 +1427,8 @@ __global__ void k_inner(const DevBlock *__restrict__ blks, const DevInner *__res
 enum HaloSet { kHaloTurb = 0, kHaloVel = 1, kHaloSpec = 2, kHaloDq = 3, kHaloEnthalpy = 4 };
 
 template <class C>
-__global__ void k_halo(const DevBlock *__restrict__ blks, const DevInner *__restrict__ faces, int fi, int set,
-                       int dq_sel) {
-  const DevInner &f = faces[fi];
+__global__ void k_halo(const DevBlock *__restrict__ blks, const DevInner *__restrict__ faces, int set, int dq_sel) {
+  const DevInner &f = faces[blockIdx.y];  // interior to ghost points: the faces are independent
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int np = f.n_point[0] * f.n_point[1] * f.n_point[2];
   if (t >= np) return;
@@ -1408,31 +1467,12 @@ __global__ void k_halo(const DevBlock *__restrict__ blks, const DevInner *__rest
   }
 }
 
-// eliminate_k_gradient, src/FieldOperation.cu:42-62 (2-D cases)
+// the 2-D plane copy alone (blockIdx.y: block)
 template <class C>
-__global__ void k_kcopy(const DevBlock *__restrict__ blks, int b) {
-  const DevBlock &B = blks[b];
-  const int g = B.ngg;
-  const int ex = B.mx + 2 * g, ey = B.my + 2 * g;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ex * ey) return;
-  const int i = t % ex - g, j = t / ex - g;
-  const int64_t sz = B.G.size, n0 = B.G.at(i, j, 0);
-  // the plane's values read once, before the stores
-  double pb[6], ps[C::nsc > 0 ? C::nsc : 1];
-  OSTC_UNROLL for (int l = 0; l < 6; ++l) pb[l] = B.bv[l * sz + n0];
-  OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) ps[l] = B.sv[l * sz + n0];
-  for (int k = 1; k <= g; ++k) {
-    const int64_t np = n0 + k * B.G.sxy, nm = n0 - k * B.G.sxy;
-    OSTC_UNROLL for (int l = 0; l < 6; ++l) {
-      B.bv[l * sz + np] = pb[l];
-      B.bv[l * sz + nm] = pb[l];
-    }
-    OSTC_UNROLL for (int l = 0; l < C::nsc; ++l) {
-      B.sv[l * sz + np] = ps[l];
-      B.sv[l * sz + nm] = ps[l];
-    }
-  }
+__global__ void k_kcopy(const DevBlock *__restrict__ blks) {
+  const DevBlock &B = blks[blockIdx.y];
+  const int g = B.ngg, ex = B.mx + 2 * g, t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < ex * (B.my + 2 * g)) copy_plane<C>(B, B.G.at(t % ex - g, t / ex - g, 0));
 }
 
 // ---------------------------------------------------------------- residual
