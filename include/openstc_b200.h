@@ -307,8 +307,9 @@ int ostc_driver_chemistry_stats(ostc_driver *d, long long *accepted, long long *
    src/Driver.cu:205-216).  schedule: the order in which the blocks of a
    multi-block grid share each launch (0 block order, 1 largest block first);
    flux_variant: on the FP32-bulk path the variant of the flux passes
-   (resident CTAs per SM and cells each thread marches over, 0-3); on the
-   FP64 path 0 the column kernel (each face evaluated once) or 1 the per-cell
+   (resident CTAs per SM and the most cells a thread marches over, 0-3); on the
+   FP64 path 0 columns or rows, by the grid (each face of a column evaluated
+   once, a row's faces one per warp) or 1 the per-cell
    kernel (each face evaluated by both of its cells, no barriers).  No choice
    changes a result. */
 typedef struct ostc_tuning {
