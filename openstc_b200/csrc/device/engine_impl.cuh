@@ -1008,6 +1008,8 @@ class EngineT final : public Engine {
   // earlier face that touches one of its points, so that every pair of faces
   // whose order could matter keeps it.  order: face indices launch by launch
   // (device), first[l]: the launch's first entry, points[l]: its largest face.
+  // A face's launch lasts 4 to 8 us whatever its size: the mixing layer's 7 faces
+  // take 3 launches (FP64 160 x 96 x 64: 79 -> 51 us).
   struct FaceLaunches {
     int *order = nullptr;
     std::vector<int> first, points;
