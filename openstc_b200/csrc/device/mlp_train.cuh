@@ -22,6 +22,7 @@
 
 #include <cuda_bf16.h>
 
+#include "stage_ring.hpp"
 #include "surrogate.hpp"
 #include "tc_mma.cuh"
 
@@ -62,6 +63,17 @@ __device__ __forceinline__ void copy_out(void *dst, const void *src, uint32_t by
                : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+// What a CTA does before it exits when one of its waits ran out: the loader
+// waits for the copies it started (`issued` chunks through the ring), the MMA
+// thread, whose last commit goes to acc, for the MMAs it issued, so that neither
+// can still reach this CTA's shared or tensor memory.
+constexpr uint32_t kDrainPolls = 1u << 20;
+template <int N>
+__device__ __forceinline__ void drain(uint64_t *full, int issued) {
+  for (int c = tc::StageRing<N>::first_open(issued); c < issued; ++c)
+    tc::mbar_wait(&full[tc::StageRing<N>::slot(c)], tc::StageRing<N>::parity(c), kDrainPolls);
 }
 
 // MN-major SWIZZLE_128B operand: 8 K rows of 64 MN elements per 1024-byte
@@ -134,6 +146,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_layer(const uint8_t *__restrict
                                                        const float *__restrict__ bias, float *z, uint8_t *out,
                                                        float *colsum, int *err) {
   constexpr int NCH = THIN ? 1 : kH / 64, KSTEPS = THIN ? 1 : 4;
+  using Ring = tc::StageRing<2>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = align1024(smem_raw);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + 2 * kStage), *done = full + 2, *acc = full + 4;
@@ -150,15 +163,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_layer(const uint8_t *__restrict
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
   bool ok = true;
+  int issued = 0;
   // BWD B operand: W as [K = its rows][N = its columns], column chunk j of
   // the image at j * rows * 128; the K chunk's rows of each
   constexpr uint32_t w_rows = THIN ? 16 : 64, w_piece = w_rows * 128;
   if (tid == 32) {  // copies
     const uint8_t *a = in + tile * NCH * kChunk;
-    for (int c = 0; c < NCH && ok; ++c) {
-      const int s = c & 1;
-      if (c >= 2) ok = tc::mbar_wait(&done[s], 0);
+    for (int c = 0; c < NCH; ++c) {
+      const int s = Ring::slot(c);
+      if (c >= 2) ok = tc::mbar_wait(&done[s], Ring::parity(c - 2));
       if (!ok) break;
+      issued = c + 1;
       uint8_t *dst = smem + s * kStage;
       expect_tx(&full[s], kChunk + (BWD ? 4 * w_piece : kH * 128));
       copy_in(dst, a + c * kChunk, kChunk, &full[s]);
@@ -171,9 +186,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_layer(const uint8_t *__restrict
     }
   } else if (tid == 0) {  // MMAs
     constexpr uint32_t idesc = tc::idesc_bf16(kTile, kH) | (BWD ? kBMn : 0u);
-    for (int c = 0; c < NCH && ok; ++c) {
-      const int s = c & 1;
-      ok = tc::mbar_wait(&full[s], (c >> 1) & 1);
+    for (int c = 0; c < NCH; ++c) {
+      const int s = Ring::slot(c);
+      ok = tc::mbar_wait(&full[s], Ring::parity(c));
       if (!ok) break;
       tc::fence_after_sync();
       const uint32_t ab = tc::smem_u32(smem + s * kStage), bb = ab + kChunk;
@@ -182,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_layer(const uint8_t *__restrict
                      idesc, (c > 0 || q > 0) ? 1u : 0u);
       if (c + 2 < NCH) tc::commit(&done[s]);
     }
-    if (ok) tc::commit(acc);
+    tc::commit(acc);  // whether or not all of them were issued
   }
   __syncwarp();
   const int row = (warp & 3) * 32 + lane, half = warp >> 2;
@@ -230,9 +245,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_layer(const uint8_t *__restrict
     if (tid == 0) copy_out(out + tile * kTileBytes, smem, kTileBytes);
     if constexpr (BWD) colsum[tile * kH + tid] = (red[tid] + red[kH + tid]) + (red[2 * kH + tid] + red[3 * kH + tid]);
   } else {
-    if (tid == 0) atomicExch(err, 1);
-    if (tid == 32)  // no copy of this CTA may still be in flight when it exits
-      for (int s = 0; s < 2 && s < NCH; ++s) tc::mbar_wait(&full[s], 0, 1u << 20);
+    if (tid == 0) {
+      atomicExch(err, 1);
+      tc::mbar_wait(acc, 0, kDrainPolls);
+    }
+    if (tid == 32) drain<2>(full, issued);
+    tc::fence_before_sync();
   }
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, kH);
@@ -276,8 +294,8 @@ __global__ void __launch_bounds__(kTile) k_out(const uint8_t *__restrict__ in, c
       for (int q = 0; q < kH / 16; ++q)
         tc::mma_bf16(tmem, tc::desc_sw128(ab + (q >> 2) * kChunk + (q & 3) * 32),
                      tc::desc_sw128(bb + (q >> 2) * 2048 + (q & 3) * 32), tc::idesc_bf16(kTile, kSurOutPad), q > 0 ? 1u : 0u);
-      tc::commit(acc);
     }
+    tc::commit(acc);
   }
   __syncwarp();
   const int64_t row = tile * kTile + tid;
@@ -332,7 +350,8 @@ __global__ void __launch_bounds__(kTile) k_out(const uint8_t *__restrict__ in, c
     }
   } else if (tid == 0) {
     atomicExch(err, 1);
-    tc::mbar_wait(full, 0, 1u << 20);
+    tc::mbar_wait(full, 0, kDrainPolls);
+    tc::mbar_wait(acc, 0, kDrainPolls);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -375,11 +394,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_dw(DwArgs a, int *err) {
   const uint32_t tmem = *tslot;
   bool ok = true;
   const int nq = thin ? 1 : 4;  // 64-column chunks of Q
+  using Ring = tc::StageRing<kDwStages>;
+  int issued = 0;
   if (tid == 32) {
-    for (int c = 0; c < nh && ok; ++c) {
-      const int s = c % kDwStages, h = h0 + c;
-      if (c >= kDwStages) ok = tc::mbar_wait(&done[s], (c / kDwStages - 1) & 1);
+    for (int c = 0; c < nh; ++c) {
+      const int s = Ring::slot(c), h = h0 + c;
+      if (c >= kDwStages) ok = tc::mbar_wait(&done[s], Ring::parity(c - kDwStages));
       if (!ok) break;
+      issued = c + 1;
       uint8_t *dst = smem + s * kDwStage;
       expect_tx(&full[s], (4 + nq) * kHalf);
       const size_t t = h >> 1, r = (h & 1) * kHalf;
@@ -389,9 +411,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_dw(DwArgs a, int *err) {
     }
   } else if (tid == 0) {
     const uint32_t idesc = tc::idesc_bf16(128, thin ? 16 : kH) | kAMn | kBMn;
-    for (int c = 0; c < nh && ok; ++c) {
-      const int s = c % kDwStages;
-      ok = tc::mbar_wait(&full[s], (c / kDwStages) & 1);
+    for (int c = 0; c < nh; ++c) {
+      const int s = Ring::slot(c);
+      ok = tc::mbar_wait(&full[s], Ring::parity(c));
       if (!ok) break;
       tc::fence_after_sync();
       const uint32_t pb = tc::smem_u32(smem + s * kDwStage), qb = pb + 4 * kHalf;
@@ -401,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dw(DwArgs a, int *err) {
                        idesc, (c > 0 || q > 0) ? 1u : 0u);
       tc::commit(&done[s]);
     }
-    if (ok) tc::commit(acc);
+    tc::commit(acc);
   }
   __syncwarp();
   ok = tc::mbar_wait(acc, 0, 1u << 26) && ok;
@@ -424,10 +446,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_dw(DwArgs a, int *err) {
       for (int e = 0; e < 16; ++e) o[(c0 + e) * kH] = v[e];
     }
   } else {
-    if (tid == 0) atomicExch(err, 1);
-    if (tid == 32)
-      for (int c = max(0, nh - kDwStages); c < nh; ++c)
-        tc::mbar_wait(&full[c % kDwStages], (c / kDwStages) & 1, 1u << 20);
+    if (tid == 0) {
+      atomicExch(err, 1);
+      tc::mbar_wait(acc, 0, kDrainPolls);
+    }
+    if (tid == 32) drain<kDwStages>(full, issued);
   }
   tc::fence_before_sync();
   __syncthreads();
