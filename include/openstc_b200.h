@@ -286,6 +286,11 @@ typedef struct ostc_surrogate_gate {
 } ostc_surrogate_gate;
 int ostc_surrogate_get_gate(const ostc_surrogate *s, ostc_surrogate_gate *g);
 int ostc_surrogate_set_gate(ostc_surrogate *s, const ostc_surrogate_gate *g);
+/* Sets the device word by which the network's kernels report a tensor-core wait
+   that ran out, without one: the next call of train (which then leaves the
+   weights alone), evaluate, predict or gradients fails as after such a wait and
+   clears it.  For tests of a program's error path. */
+int ostc_surrogate_mark_timeout(ostc_surrogate *s);
 int ostc_surrogate_save(const ostc_surrogate *s, const char *path);
 int ostc_surrogate_load(ostc_surrogate *s, const char *path);
 /* Chemistry of the driver's steps through the surrogate.  Before the source

@@ -151,6 +151,7 @@ def library() -> C.CDLL:
         "ostc_surrogate_get_params": ([P, P], C.c_int),
         "ostc_surrogate_set_params": ([P, P], C.c_int),
         "ostc_surrogate_normalisation": ([P, P, P, P, P], C.c_int),
+        "ostc_surrogate_mark_timeout": ([P], C.c_int),
         "ostc_surrogate_save": ([P, C.c_char_p], C.c_int),
         "ostc_surrogate_load": ([P, C.c_char_p], C.c_int),
         "ostc_driver_set_surrogate": ([P, P], C.c_int),

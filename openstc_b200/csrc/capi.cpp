@@ -613,6 +613,14 @@ int ostc_surrogate_set_gate(ostc_surrogate *s, const ostc_surrogate_gate *g) {
   return OSTC_OK;
 }
 
+int ostc_surrogate_mark_timeout(ostc_surrogate *s) {
+  if (!s) return fail(OSTC_ERR_INPUT, "null argument");
+  return guarded([&] {
+    s->s->mark_timeout();
+    return OSTC_OK;
+  });
+}
+
 int ostc_surrogate_save(const ostc_surrogate *s, const char *path) {
   if (!s || !path) return fail(OSTC_ERR_INPUT, "null argument");
   return guarded([&] {

@@ -458,7 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_dw(DwArgs a, int *err) {
 }
 
 // Sums the partial gradients and takes the Adam step (grad null), or stores
-// the gradient in the flat parameter order (per layer W, then b).  Blocks of
+// the gradient in the flat parameter order (per layer W, then b); nothing after
+// a wait that ran out, so that the weights stay those of the last whole step.  Blocks of
 // 32 x 8 threads: kWeightBlocks tiles of 32 x 32 weights, then 32 bias columns
 // each, then the loss.
 struct StepArgs {
@@ -469,6 +470,7 @@ struct StepArgs {
   const double *loss_part;
   double *loss;
   float *grad;
+  const int *err;  // not 0: a wait of an earlier kernel ran out, its results are not there
   float lr, b1, b2, eps, bc1, bc2;
 };
 constexpr int kThinBlocks = kH / 32, kHiddenBlocks = kThinBlocks * kThinBlocks;
@@ -491,6 +493,7 @@ __device__ __forceinline__ int flat_offset(int layer, bool bias) {
 }
 
 __global__ void __launch_bounds__(256) k_step(StepArgs a) {
+  if (*a.err) return;
   __shared__ float tile[32][33];
   const int x = threadIdx.x, y = threadIdx.y;
   int blk = blockIdx.x;

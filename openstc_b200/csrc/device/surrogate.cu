@@ -533,6 +533,7 @@ void Surrogate::reduce(float *grad, double lr, double *loss) {
   a.loss_part = loss_part_;
   a.loss = loss;
   a.grad = grad;
+  a.err = err_;
   a.lr = static_cast<float>(lr);
   a.b1 = 0.9f;
   a.b2 = 0.999f;
@@ -541,6 +542,21 @@ void Surrogate::reduce(float *grad, double lr, double *loss) {
   a.bc2 = 1.f - std::pow(a.b2, static_cast<float>(adam_t_));
   mlp::k_step<<<mlp::kStepBlocks, dim3(32, 8), 0, stream_>>>(a);
   ck(cudaGetLastError(), "gradient step");
+}
+
+// Throws if a wait of the kernels since the last check ran out, and starts
+// afresh.
+void Surrogate::check_waits(const char *what) {
+  int err = 0;
+  d2h(&err, err_, sizeof(int), "err copy");
+  if (!err) return;
+  ck(cudaMemsetAsync(err_, 0, sizeof(int), stream_), "err");
+  throw std::runtime_error(std::string("tensor-core wait timed out during ") + what);
+}
+
+void Surrogate::mark_timeout() {
+  ck(cudaSetDevice(device_), "cudaSetDevice");
+  ck(cudaMemsetAsync(err_, 1, sizeof(int), stream_), "err");
 }
 
 double Surrogate::train(int steps, int batch, double lr, int64_t n_train, float *losses) {
@@ -552,6 +568,9 @@ double Surrogate::train(int steps, int batch, double lr, int64_t n_train, float 
   // synchronisation between steps
   DevTemp<double> dloss_buf(static_cast<size_t>(std::max(1, steps)), "cudaMalloc losses");
   double *dloss = dloss_buf.p;
+  // all bits set, a NaN that no sum gives: the steps not taken after a timeout
+  ck(cudaMemsetAsync(dloss, 0xff, sizeof(double) * static_cast<size_t>(std::max(1, steps)), stream_), "losses");
+  const int first = adam_t_;
   for (int s = 0; s < steps; ++s) {
     gather(x_, t_, n_train, mix64(seed_ + 0x5151 * (adam_t_ + 1)), false);
     forward(true);
@@ -570,11 +589,14 @@ double Surrogate::train(int steps, int batch, double lr, int64_t n_train, float 
   ck(st, "train steps");
   if (losses)
     for (int s = 0; s < steps; ++s) losses[s] = static_cast<float>(hl[s]);
-  const double last = steps > 0 ? hl[steps - 1] : 0.0;
-  int err = 0;
-  d2h(&err, err_, sizeof(int), "err copy");
-  if (err) throw std::runtime_error("tensor-core wait timed out during training");
-  return last;
+  int taken = 0;
+  for (uint64_t bits = 0; taken < steps; ++taken) {
+    std::memcpy(&bits, &hl[taken], sizeof(bits));
+    if (bits == ~0ull) break;
+  }
+  adam_t_ = first + taken;
+  check_waits("training");
+  return steps > 0 ? hl[steps - 1] : 0.0;
 }
 
 std::vector<std::vector<float>> Surrogate::params() const {
@@ -664,6 +686,7 @@ void Surrogate::predict_host(const double *states, int64_t n, double *dy, int *a
   ck(cudaMemcpyAsync(dy, d, n * NS * 8, cudaMemcpyDeviceToHost, stream_), "predict download");
   ck(cudaMemcpyAsync(accepted, acc, n * sizeof(int), cudaMemcpyDeviceToHost, stream_), "predict download");
   ck(cudaStreamSynchronize(stream_), "predict");
+  check_waits("prediction");
 }
 
 double Surrogate::grad_host(const double *states, const double *dy, int64_t n, std::vector<std::vector<float>> &grads) {
@@ -694,6 +717,7 @@ double Surrogate::grad_host(const double *states, const double *dy, int64_t n, s
   double loss = 0;
   ck(cudaMemcpyAsync(&loss, loss_, sizeof(double), cudaMemcpyDeviceToHost, stream_), "loss");
   ck(cudaStreamSynchronize(stream_), "grad");
+  check_waits("the gradients");
   return loss;
 }
 

@@ -100,6 +100,8 @@ class Surrogate {
   void save(const std::string &path) const;
   void load(const std::string &path);
   const SurrogateDev &device_params();  // packed for the fused kernel
+  // As if a tensor-core wait of the next call's kernels ran out (tests).
+  void mark_timeout();
   int device() const { return device_; }
   cudaStream_t stream() const { return stream_; }
   // the normalisation (features and targets)
@@ -115,6 +117,7 @@ class Surrogate {
   void output_layer(bool train);
   void backward();
   void reduce(float *grad, double lr, double *loss);
+  void check_waits(const char *what);
   void pack();
   void upload_chem();
   void launch_label(const double *states, double *dy, int64_t n);

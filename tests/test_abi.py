@@ -176,6 +176,7 @@ def test_surrogate_entry_points_refuse_a_null_handle():
         "ostc_surrogate_load": (b"never_read.bin",),
         "ostc_surrogate_get_gate": (ctypes.byref(gate),),
         "ostc_surrogate_set_gate": (ctypes.byref(gate),),
+        "ostc_surrogate_mark_timeout": (),
     }
     for name, args in calls.items():
         assert getattr(lib, name)(None, *args) == -1, name  # OSTC_ERR_INPUT

@@ -281,3 +281,29 @@ def test_what_the_network_gains(trained, tmp_path):
     assert accepted + fallback == steps * runs["fp64"]["T"].size
     assert accepted > 0
     print(f"network took {accepted / (accepted + fallback):.3f} of the cell-steps' chemistry")
+
+
+def test_a_timed_out_wait_is_reported_by_every_call(drv):
+    """The word the kernels set when a tensor-core wait runs out (set here by
+    the test): no call returns what lay in the buffers before, training takes no
+    step from them, and the next call works again."""
+    sur, twin = ostc.Surrogate(drv, seed=11), ostc.Surrogate(drv, seed=11)
+    for s in (sur, twin):
+        s.generate(4096, seed=2)
+        s.train(2, batch=1024)
+    st = random_states(256, 14)
+    dy = sur.label(st)
+    good = sur.predict(st)
+    before = sur.params()
+    calls = [lambda: sur.train(3, batch=1024), lambda: sur.predict(st), lambda: sur.gradients(st, dy),
+             lambda: sur.evaluate(0, 512)]
+    for call in calls:
+        assert ostc.library().ostc_surrogate_mark_timeout(sur._h) == 0
+        with pytest.raises(ostc.OstcError, match="timed out"):
+            call()
+        assert np.array_equal(sur.params(), before)
+        call_again = sur.predict(st)
+        assert np.array_equal(call_again[0], good[0]) and np.array_equal(call_again[1], good[1])
+    # weights, moments and step count are those of a surrogate that saw none of it
+    assert np.array_equal(sur.train(2, batch=1024), twin.train(2, batch=1024))
+    assert np.array_equal(sur.params(), twin.params())
