@@ -16,6 +16,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "known_divisor.hpp"
 
 namespace ostc {
 
@@ -37,19 +38,9 @@ struct Cfg {
 
 __device__ __forceinline__ double ld(const double *p) { return __ldg(p); }
 
-// x / y for a divisor known in advance, with 1 / y = zh + zl: two operations
-// instead of a division (N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
-// correctly rounded floating-point division when the divisor is known in
-// advance", IEEE Trans. Computers 53, 2004).  The quotient is the correctly
-// rounded one unless x / y lies within about 2^-100 of the middle between two
-// doubles (x neither infinite nor so small that x zl underflows).  The FP64 path
-// divides by W_k and by 3 some 150 times per cell and step.
-__device__ __forceinline__ double div_by(double x, double zh, double zl) {
-  return __fma_rn(x, zh, __dmul_rn(x, zl));
-}
 __device__ __forceinline__ double div_mw(double x, int l) { return div_by(x, cP.mw_h[l], cP.mw_l[l]); }
 __device__ __forceinline__ double div_3(double x) {
-  constexpr double zh = 1.0 / 3.0, zl = 1.850371707708594e-17;  // 1 / 3 - zh
+  constexpr double zh = 1.0 / 3.0, zl = 1.850371707708594e-17;  // reciprocal(3)
   return div_by(x, zh, zl);
 }
 

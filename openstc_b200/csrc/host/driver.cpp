@@ -13,6 +13,7 @@
 #include <mutex>
 #include <thread>
 
+#include "../device/known_divisor.hpp"
 #include "plt_io.hpp"
 
 namespace ostc {
@@ -288,8 +289,9 @@ void Driver::build_dev_params() {
   for (int i = 0; i < ns; ++i) {
     p.mw[i] = spec.mw[i];
     p.ru_mw[i] = kRu / spec.mw[i];
-    p.mw_h[i] = 1.0 / spec.mw[i];
-    p.mw_l[i] = std::fma(-p.mw_h[i], spec.mw[i], 1.0) / spec.mw[i];
+    const Reciprocal z = reciprocal(spec.mw[i]);
+    p.mw_h[i] = z.h;
+    p.mw_l[i] = z.l;
     p.t_low[i] = spec.t_low[i];
     p.t_mid[i] = spec.t_mid[i];
     for (int q = 0; q < 7; ++q) {

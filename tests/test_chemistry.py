@@ -3,6 +3,12 @@
 The reference ships no tests; these pin the parse of its own mechanism
 (input_files/chemistry) and physical invariants of the oracle's chemistry."""
 import ctypes as C
+import math
+import random
+import struct
+import subprocess
+from fractions import Fraction as F
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -149,24 +155,80 @@ def test_compile_time_mechanism_is_the_shipped_one(params):
     assert table("sb[nr][ns]") == list(params.stoi_b[:19 * 9])
 
 
-def test_division_by_known_divisors_is_correctly_rounded(params):
-    """div_by (physics.cuh) with 1 / y as the sum of two doubles gives x / y for
-    the divisors the FP64 path uses it for, the molecular weights and 3, over the
-    exponents its operands have: exact rational arithmetic stands in for the
-    fused multiply-add."""
-    import random
-    from fractions import Fraction as F
+@pytest.fixture(scope="module")
+def quotients(tmp_path_factory):
+    """quotients(y, xs): the two parts of 1 / y and div_by of every x."""
+    d = tmp_path_factory.mktemp("div")
+    (d / "div.cpp").write_text("""
+#include <cstdio>
+#include <cstdlib>
+#include "device/known_divisor.hpp"
+int main(int, char **argv) {
+  const ostc::Reciprocal z = ostc::reciprocal(std::strtod(argv[1], nullptr));
+  std::printf("%a %a\\n", z.h, z.l);
+  char text[64];
+  while (std::scanf("%63s", text) == 1) std::printf("%a\\n", ostc::div_by(std::strtod(text, nullptr), z.h, z.l));
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-ffp-contract=off", "-I", str(Path(ostc.__file__).parent / "csrc"),
+                    str(d / "div.cpp"), "-o", str(d / "div")], check=True)
 
-    def fma(a, b, c):
-        return float(F(a) * F(b) + F(c))
+    def run(y, xs):
+        out = subprocess.run([str(d / "div"), y.hex()], input="\n".join(float(x).hex() for x in xs),
+                             capture_output=True, text=True, check=True).stdout.split()
+        v = [float.fromhex(t) for t in out]
+        return v[:2], v[2:]
 
+    return run
+
+
+def near_middles(y, widest=64):
+    """Every significand x whose quotient x / y lies within widest 2^-106 of the
+    middle between two doubles, in units of the quotient: x 2^s - (odd) y = d has
+    one x for each small d, modulo the odd part of y's significand."""
+    Y = int(math.frexp(y)[0] * 2 ** 53)
+    t = (Y & -Y).bit_length() - 1
+    odd = Y >> t
+    xs = []
+    if widest >> t == 0:
+        return xs  # no d but 0, and no quotient of doubles is a middle
+    for s in (53, 54):  # x >= Y: quotient in [1, 2); x < Y: in [1/2, 1)
+        for e in range(-(widest >> t), (widest >> t) + 1):
+            x = e * pow(2, -(s - t), odd) % odd
+            while x < 2 ** 53:
+                if x >= 2 ** 52 and (x >= Y) == (s == 53) and (x * 2 ** s - (e << t)) // Y % 2 == 1:
+                    xs.append(float(x))
+                x += odd
+    return xs
+
+
+def test_division_by_known_divisors_is_the_division(params, quotients):
+    """div_by (known_divisor.hpp) gives the bits of x / y for the divisors the FP64
+    path uses it for, the molecular weights and 3, and for powers of two: over
+    the exponents its operands have, at the quotients nearest to the middle
+    between two doubles, and for zeros, infinities and NaN."""
     rng = random.Random(7)
-    for y in [3.0] + list(params.mw[:9]):
-        zh = 1.0 / y
-        zl = fma(-zh, y, 1.0) / y
+    special = [0.0, -0.0, math.inf, -math.inf, math.nan, 1.7e308, -1.7e308]
+    for y in [3.0, 2.0, 16.0] + list(params.mw[:9]):
+        xs = [rng.choice([-1, 1]) * rng.uniform(1, 2) * 2.0 ** rng.randint(-950, 1020) for _ in range(2000)]
+        hard = near_middles(y)
+        assert len(hard) > 20 or y in (3.0, 2.0, 16.0)
+        xs += special + hard + [-x for x in hard]
+        (h, l), got = quotients(y, xs)
+        assert l > 0 and abs(F(h) + F(l) - 1 / F(y)) < F(2) ** -104 / F(y)
         if y == 3.0:
-            assert zl == 1.850371707708594e-17  # the header's literal
-        for _ in range(500):
-            x = rng.choice([-1, 1]) * rng.uniform(1, 2) * 2.0 ** rng.randint(-200, 200)
-            assert fma(x, zh, x * zl) == x / y, (x, y)
-        assert fma(0.0, zh, 0.0 * zl) == 0.0
+            assert (h, l) == (1.0 / 3.0, 1.850371707708594e-17)  # the literals of div_3
+        want = [x / y for x in xs]
+        wrong = [x for x, a, b in zip(xs, got, want) if struct.pack("d", a) != struct.pack("d", b) and x == x]
+        assert not wrong, (y, [x.hex() for x in wrong[:5]])
+        assert math.isnan(got[2000 + special.index(special[4])])
+
+
+def test_division_of_the_smallest_numbers_is_one_double_off_at_most(params, quotients):
+    """Below 2^-960 x zl underflows: the quotient or the double beside it."""
+    rng = random.Random(8)
+    for y in [3.0] + list(params.mw[:9]):
+        xs = [rng.uniform(1, 2) * 2.0 ** rng.randint(-1074, -960) for _ in range(2000)] + [5e-324, 2.3e-308]
+        _, got = quotients(y, xs)
+        for x, q in zip(xs, got):
+            assert abs(F(q) - F(x / y)) <= F(math.ulp(x / y)), (y, x)
