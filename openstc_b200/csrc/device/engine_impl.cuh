@@ -102,6 +102,11 @@ class EngineT final : public Engine {
       cuda_check(cudaFuncSetAttribute(k_flux_col<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(col_smem_)),
                  "column flux smem");
+    if constexpr (!C::mixed) {
+      if (row_smem<C>() > 48 * 1024)
+        cuda_check(cudaFuncSetAttribute(k_flux_row<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, row_smem<C>()),
+                   "row flux smem");
+    }
     if (source_smem_ > 48 * 1024) {
       if constexpr (C::mixed) {
         cuda_check(cudaFuncSetAttribute(source_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -735,17 +740,17 @@ class EngineT final : public Engine {
   // the case has its stoichiometry, the general loops otherwise.  Source stage
   // at 160 x 96 x 64, general and unrolled: FP64 2.23 and 1.12 ms, FP32-bulk
   // path 1.06 and 0.39 ms (one B200).
-  bool fixed_mechanism() const { return C::mix == 2 && mech::matches<mech::H2O2>(setup_.params); }
+  using Fixed = std::conditional_t<C::mix == 2 && C::ns == mech::H2O2::ns, mech::H2O2, void>;
+  bool fixed_mechanism() const { return !std::is_void_v<Fixed> && mech::matches<mech::H2O2>(setup_.params); }
 
   auto source_kernel() const {
-    using Fixed = std::conditional_t<C::mix == 2, mech::H2O2, void>;
     if constexpr (C::mixed)
       return fixed_mechanism() ? k_source_mx<C, Fixed> : k_source_mx<C, void>;
     else
       return fixed_mechanism() ? k_source<C, Fixed> : k_source<C, void>;
   }
 
-  auto chem_list_kernel() const { return fixed_mechanism() ? k_chem_list<C, mech::H2O2> : k_chem_list<C, void>; }
+  auto chem_list_kernel() const { return fixed_mechanism() ? k_chem_list<C, Fixed> : k_chem_list<C, void>; }
 
   void launch_source() {
     if constexpr (C::mixed) {
@@ -787,7 +792,7 @@ class EngineT final : public Engine {
       // the per-cell form: each face evaluated by both of its cells, no barriers
       k_flux<C><<<grid(tiles0_), block3(), flux_smem_, stream_>>>(d_blocks_, tiles0_, fresh);
     } else if (row_warps_ > 0) {
-      k_flux_row<C><<<grid(col_tiles_), dim3(32, row_warps_), 0, stream_>>>(d_blocks_, col_tiles_, fresh);
+      k_flux_row<C><<<grid(col_tiles_), dim3(32, row_warps_), row_smem<C>(), stream_>>>(d_blocks_, col_tiles_, fresh);
     } else {
       k_flux_col<C><<<grid(col_tiles_), kFluxThreads, col_smem_, stream_>>>(d_blocks_, col_tiles_, col_kc_, fresh);
     }

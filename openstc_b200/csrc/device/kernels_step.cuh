@@ -341,11 +341,17 @@ __global__ void __launch_bounds__(kFluxThreads, 2) k_flux_col(const DevBlock *__
 // instead of 652, the 48 x 24 ramp 12 us instead of 19.
 constexpr int kRowFaces = 6;
 
+// every face of a row of 32 cells: 48 KB for 16 variables
+template <class C>
+constexpr int row_smem() {
+  return 2 * kRowFaces * C::nv * 32 * static_cast<int>(sizeof(double));
+}
+
 template <class C>
 __global__ void __launch_bounds__(2 * kRowFaces * 32, C::mix == 0 ? 2 : 1)
     k_flux_row(const DevBlock *__restrict__ blks, Tiles T, bool fresh) {
   constexpr int NV = C::nv;
-  __shared__ double sm[2 * kRowFaces * NV * 32];
+  extern __shared__ double sm[];  // row_smem<C>()
   int b;
   int t = tile_of(T, blockIdx.x, b);
   const int tx = t % T.ntx[b];
@@ -582,12 +588,12 @@ __device__ __forceinline__ void dq0_epi(const DevBlock &B, int64_t nz, int64_t s
 // the stores to shared memory, one memory latency each).
 template <int N, int R>
 __device__ __forceinline__ void copy_slice_batched(double *slice, const double *src, int64_t st) {
-  static_assert(N % R == 0);
   OSTC_UNROLL for (int q = 0; q < N; q += R) {
     double v[R];
     OSTC_UNROLL for (int e = 0; e < R; ++e)
-      asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[e]) : "l"(src + (q + e) * st) : "memory");
-    OSTC_UNROLL for (int e = 0; e < R; ++e) slice[(q + e) * kCta] = v[e];
+      if (q + e < N) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[e]) : "l"(src + (q + e) * st) : "memory");
+    OSTC_UNROLL for (int e = 0; e < R; ++e)
+      if (q + e < N) slice[(q + e) * kCta] = v[e];
   }
 }
 
