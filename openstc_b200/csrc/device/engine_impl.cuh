@@ -22,6 +22,7 @@ class EngineT final : public Engine {
  public:
   explicit EngineT(const EngineSetup &s) : setup_(s) {
     cuda_check(cudaSetDevice(s.device), "cudaSetDevice");
+    cuda_check(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, s.device), "SM count");
     cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     if (s.params.ns != C::ns) throw std::runtime_error("engine instantiated for another species count");
     if (static_cast<int>(s.dims.size()) > kMaxBlocks)
@@ -921,8 +922,6 @@ class EngineT final : public Engine {
                          sur::k_sur_infer<C, 1, 4>})
           cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sur::kSmem)),
                      "surrogate smem");
-        // the persistent inference kernel runs one CTA per SM
-        cuda_check(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, setup_.device), "SM count");
         const int fb_smem = static_cast<int>(2 * std::max(1, setup_.params.nr) * 128 * sizeof(double));
         if (fb_smem > 48 * 1024)
           cuda_check(cudaFuncSetAttribute(sur::k_sur_fallback<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb_smem),
@@ -1346,7 +1345,7 @@ class EngineT final : public Engine {
   cudaGraphExec_t graphs_[4] = {nullptr, nullptr, nullptr, nullptr};
   bool sur_on_ = false;
   SurrogateDev sur_{};
-  int num_sms_ = 148;
+  int num_sms_ = 0;  // of the device; the cuts of the launches follow it
   int *d_fb_count_ = nullptr, *d_fb_list_ = nullptr, *d_sur_err_ = nullptr, *d_sur_phase_ = nullptr;
   unsigned long long *d_sur_stats_ = nullptr;
   std::vector<void *> sur_arrays_;
