@@ -846,6 +846,10 @@ class EngineT final : public Engine {
 
   void launch_residual() {
     if (sur_on_) launch_classify();
+    launch_rhs();
+  }
+
+  void launch_rhs() {
     constexpr bool no_source = C::mix != 2 && !C::turb;  // the source stage would only zero dq
     if constexpr (!no_source) {
       launch_source();
@@ -1289,11 +1293,8 @@ class EngineT final : public Engine {
 
   double time_stages(int reps) override {
     upload_params();
-    auto pass = [this] {
-      launch_source();
-      launch_halo(kHaloTurb);
-      launch_flux();
-      launch_halo(kHaloSpec);
+    auto pass = [this] {  // the step's stages that the tunings change
+      launch_rhs();
       launch_implicit();
     };
     pass();
