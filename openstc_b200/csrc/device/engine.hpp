@@ -106,7 +106,7 @@ class Engine {
 
   // Tuning.  schedule: the order of the blocks in every launch (0 block
   // order, 1 largest block first); flux_variant: the variant of the FP32-bulk
-  // flux passes (fp32 kFluxVariant; 0 on the FP64 path).  Neither changes a
+  // flux passes (kFluxVariant), on the FP64 path 0 columns or rows, 1 per cell.  Neither changes a
   // result.  Drops the captured step graphs.
   virtual void set_tuning(int schedule, int flux_variant) = 0;
   virtual int flux_variants() const = 0;

@@ -630,90 +630,38 @@ class EngineT final : public Engine {
     return t;
   }
 
-  // the tiles of direction pass d of the FP32-bulk flux (dir_tile_counts)
-  Tiles make_dir_tiles(int d, int march) const {
-    return build_tiles([d, march](const DevBlock &B, int &ntx, int &nty) {
-      int n2 = 0;
-      dir_tile_counts(d, march, B.mx, B.my, B.mz, ntx, nty, n2);
-      return ntx * nty * n2;
+  // the tiles of a flux launch: `cut` of every block (flux_cut.hpp)
+  template <class Cut>
+  Tiles make_cut_tiles(Cut &&cut) const {
+    return build_tiles([&cut](const DevBlock &B, int &ntx, int &nty) {
+      const BlockDims t = cut(BlockDims{B.mx, B.my, B.mz});
+      ntx = t[0];
+      nty = t[1];
+      return t[0] * t[1] * t[2];
     });
   }
 
-  // columns of kTX x kTY cells over kc planes (the k-marching flux kernel)
-  Tiles make_col_tiles(int kc) const {
-    return build_tiles([kc](const DevBlock &B, int &ntx, int &nty) {
-      ntx = (B.mx + kTX - 1) / kTX;
-      nty = (B.my + kTY - 1) / kTY;
-      return ntx * nty * ((B.mz + kc - 1) / kc);
-    });
-  }
-
-  // rows of 32 cells (k_flux_row)
-  Tiles make_row_tiles() const {
-    return build_tiles([](const DevBlock &B, int &ntx, int &nty) {
-      ntx = (B.mx + 31) / 32;
-      nty = B.my;
-      return ntx * nty * B.mz;
-    });
-  }
-
-  // The time of a flux launch in units of one face evaluation on an idle SM:
-  // a thread evaluates `serial` faces one after another, which take up to 1 + a
-  // times as long once every slot (SMs x resident CTAs) is taken, and waves of
-  // CTAs follow each other (a wave's end overlaps the next one by about half).
-  static double flux_cost(double serial, int ctas, int slots, double a) {
-    const double w = static_cast<double>(ctas) / slots;
-    return serial * (1 + a * std::min(1.0, w)) * (w <= 1 ? 1.0 : 0.5 * (w + std::ceil(w)));
-  }
-
-  // How the flux kernels cut the grid.  Long columns or marches evaluate the
-  // fewest faces, short ones keep the SMs of a small grid busy; the constants
-  // are from event times on one B200.  FP64 (reacting layer, in us; taken
-  // before the divisions by constants became products (div_by), which made a
-  // full grid 17 % faster: 160 x 96 x 64 is 2.7 ms now; the order is the same):
-  //   24 x 16 x 8:    8 / 4 / 2 / 1 planes 652 / 344 / 190 / 112, rows 24
-  //   45 x 37 x 21:                        707 / 381 / 225 / 240, rows 217
-  //   96 x 64 x 32:                        909 / 872 / 724 / 768, rows 868
-  //   160 x 96 x 64:                     3432 / 3291 / 3328 / 3537, rows 4199
-  // laminar ramp (columns, rows): 128 x 64 21, 11; 256 x 128 21, 25.
-  // FP32-bulk, y pass (march 8 / 4 / 2 / 1):
-  //   24 x 16 x 8: 153 / 88 / 54 / 39     96 x 64 x 32: 222 / 141 / 102 / 131
-  //   160 x 96 x 64: 336 / 364 / 412 / 457
   void make_flux_tiles() {
+    std::vector<BlockDims> dims;
+    bool three_d = false;
+    for (const auto &B : blocks_) {
+      dims.push_back({B.mx, B.my, B.mz});
+      three_d = three_d || B.mz > 1;
+    }
     if constexpr (C::mixed) {
-      const FluxVariant v = kFluxVariant[flux_variant_];
-      dir_tiles_[0] = make_dir_tiles(0, 1);
-      for (int d = 1; d < 3; ++d) {
-        double best = 0;
-        for (int m = v.march; m >= 1; m /= 2) {
-          const Tiles t = make_dir_tiles(d, m);
-          const double cost = flux_cost(m + 1, t.begin[t.nblk], num_sms_ * v.min_blocks, 1.25);
-          if (m < v.march && cost >= best) continue;
-          best = cost;
-          march_[d] = m;
-          dir_tiles_[d] = t;
-        }
+      for (int d = 0; d < 3; ++d) {
+        const int m = d == 0 ? 1 : march_cut(dims, d, kFluxVariant[flux_variant_], num_sms_);
+        march_[d] = m;
+        dir_tiles_[d] = make_cut_tiles([d, m](const BlockDims &b) { return dir_tile_counts(d, m, b); });
       }
     } else {
-      bool three_d = false;
-      for (const auto &B : blocks_) three_d = three_d || B.mz > 1;
-      double best = 0;
-      for (int kc = three_d ? kFluxKC : 1; kc >= 1; kc /= 2) {
-        const Tiles t = make_col_tiles(kc);
-        const double cost = flux_cost(three_d ? 6 * kc + 2 : 4, t.begin[t.nblk], 2 * num_sms_, 0.35);
-        if (best > 0 && cost >= best) continue;
-        best = cost;
-        col_kc_ = kc;
-        col_tiles_ = t;
-      }
-      const Tiles t = make_row_tiles();
-      const double cost =
-          flux_cost(1.5, t.begin[t.nblk], (C::mix == 0 ? 2 : 1) * num_sms_, 0) + (three_d ? 0.0 : 0.9);
-      row_warps_ = 0;
-      if (cost < best) {
-        row_warps_ = 2 * (three_d ? kRowFaces : kRowFaces - 2);
-        col_tiles_ = t;
-      }
+      const Fp64Cut cut = fp64_flux_cut(dims, num_sms_, C::mix == 0);
+      row_warps_ = cut.rows ? 2 * (three_d ? kRowFaces : kRowFaces - 2) : 0;
+      col_kc_ = cut.kc;
+      if (cut.rows)
+        col_tiles_ = make_cut_tiles(row_tile_counts);
+      else
+        col_tiles_ = make_cut_tiles([&cut](const BlockDims &b) { return col_tile_counts(cut.kc, b); });
     }
   }
 

@@ -651,38 +651,9 @@ __device__ __forceinline__ void local_time_step_q(const DevBlock &B, const float
 //   y, z: each thread marches over some cells along d, carrying the lower face
 //      from one cell to the next; lanes run along i, the CTA's 4 warps over
 //      the remaining index (k for y, j for z).
-constexpr int kXSeg = 31;  // cells per warp of the x pass
-// The variants of the passes an autotuner chooses from: resident CTAs per
-// SM the register allocator is asked to allow (8 caps a thread at 64
-// registers, ~400 B of spills) and the cells a thread of the y / z pass
-// marches over at most (fewer where the grid would leave SMs idle).  Measured at 384x192x64 with a march of 8, the three passes
-// take 5.7 ms at 4 CTAs per SM, 5.0 at 6, 4.8 at 7, 4.4 at 8.  Every variant
-// computes the same values.
-struct FluxVariant {
-  int min_blocks, march;
-};
-constexpr int kFluxVariants = 4;
-constexpr FluxVariant kFluxVariant[kFluxVariants] = {{8, 8}, {8, 16}, {6, 8}, {4, 8}};
-
-// Tiles of pass d over every block: (x) i-segments x row groups x k,
-// (y) i-groups x k-groups x j-segments, (z) i-groups x j-groups x k-segments
-// of `march` cells.
-inline void dir_tile_counts(int d, int march, int mx, int my, int mz, int &n0, int &n1, int &n2) {
-  if (d == 0) {
-    n0 = (mx + kXSeg - 1) / kXSeg;
-    n1 = (my + kTY - 1) / kTY;
-    n2 = mz;
-  } else if (d == 1) {
-    n0 = (mx + kTX - 1) / kTX;
-    n1 = (mz + kTY - 1) / kTY;
-    n2 = (my + march - 1) / march;
-  } else {
-    n0 = (mx + kTX - 1) / kTX;
-    n1 = (my + kTY - 1) / kTY;
-    n2 = (mz + march - 1) / march;
-  }
-}
-
+// The variants (flux_cut.hpp) differ in registers: 8 CTAs per SM cap a thread at 64
+// registers, ~400 B of spills.  Measured at 384x192x64 with a march of 8, the three
+// passes take 5.7 ms at 4 CTAs per SM, 5.0 at 6, 4.8 at 7, 4.4 at 8.
 __device__ __forceinline__ void dir_tile(const Tiles &T, int &b, int &t0, int &t1, int &t2) {
   int t = tile_of(T, blockIdx.x, b);
   t0 = t % T.ntx[b];

@@ -1,11 +1,11 @@
 // Kernels of one pseudo-time step, instantiated per model configuration.
 #pragma once
 
+#include "flux_cut.hpp"
 #include "kernels.cuh"
 
 namespace ostc {
 
-constexpr int kTX = 32, kTY = 4, kTZ = 1;  // per-cell tile (threads)
 constexpr int kCta = kTX * kTY * kTZ;
 
 // ---------------------------------------------------------------- source
@@ -192,7 +192,6 @@ __global__ void __launch_bounds__(kCta, OSTC_FLUX_MIN_BLOCKS) k_flux(const DevBl
 // same order (dq -= f(+) - f(-) per direction, inviscid then viscous), so the
 // result is bit-identical.  The planes per column (kc, at most kFluxKC) are
 // chosen by the launch.
-constexpr int kFluxKC = 8;                  // k planes per column at most
 constexpr int kFluxThreads = kCta + 32;     // 4 compute warps + the minus-face warp
 
 __device__ __forceinline__ void col_tile(const Tiles &T, int kc, int &b, int &i0, int &j0, int &k0) {

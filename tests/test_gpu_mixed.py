@@ -66,11 +66,11 @@ FLUX_INPUTS = ("bv", "sv", "mul", "conductivity", "rho_d", "gamma", "cp", "mut",
                "mach")
 
 
-@pytest.mark.parametrize("shape", [(40, 10, 11), (24, 16, 8)])
+@pytest.mark.parametrize("shape", [(40, 10, 11), (24, 16, 8), (97, 61, 31)])
 def test_mixed_flux_matches_fp64_flux(case_factory, shape):
-    """The FP32 column flux (primitive stencil staged in shared memory) against
-    the FP64 flux on the same state, at sizes that leave partial columns in
-    i, j and k: the flux differences added to dq within 1e-3 relative L2 per
+    """The direction passes of the FP32-bulk flux against the FP64 flux on the same
+    state, at sizes that leave partial warps and marches in i, j and k (marches of
+    one cell on the small grids, of two on the last): the flux differences added to dq within 1e-3 relative L2 per
     equation (an indexing fault gives O(1)), the local time step within 1e-5."""
     mx, my, mz = shape
     case = case_factory("mixed_flux", cases.mixing_layer_case, mx=mx, my=my, mz=mz, total_step=3,

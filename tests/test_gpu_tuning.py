@@ -7,6 +7,7 @@ import pytest
 
 import openstc_b200 as ostc
 from openstc_b200 import cases
+from flux_cuts import FP64_GRIDS, MIXED_GRIDS
 
 pytestmark = pytest.mark.gpu
 
@@ -94,6 +95,22 @@ def test_grid_dependent_cuts_give_the_same_fluxes(case_factory, precision, dims)
         fields = ("bv", "sv", "dq", "dt_local")
     ref, _ = run(case, precision, 0, 1, steps=2, fields=fields)
     for variant in (0,) if precision == "fp64" else (0, 2, 3):
+        got, _ = run(case, precision, 0, variant, steps=2, fields=fields)
+        for f in fields:
+            assert np.array_equal(got[f][0], ref[f][0], equal_nan=True), (variant, f)
+
+
+@pytest.mark.parametrize("precision,dims", [("fp64", g) for g in FP64_GRIDS] + [("mixed", g) for g in MIXED_GRIDS])
+def test_every_cut_gives_the_same_fluxes(tmp_path, precision, dims):
+    """Columns of 1, 2, 4 and 8 planes and rows against the per-cell kernel, and
+    marches of 1, 2, 4, 8 and 16 cells along y and z against each other, with last
+    segments that are not full (test_flux_cuts.py says which grid takes which): dq
+    and the time step bit for bit."""
+    mx, my, mz = dims
+    case = cases.mixing_layer_case(tmp_path / "c", mx=mx, my=my, mz=mz, total_step=2, output_screen=1)
+    fields = ("dq", "dt_local")
+    ref, _ = run(case, precision, 0, 0, steps=2, fields=fields)
+    for variant in (1,) if precision == "fp64" else (1, 2, 3):
         got, _ = run(case, precision, 0, variant, steps=2, fields=fields)
         for f in fields:
             assert np.array_equal(got[f][0], ref[f][0], equal_nan=True), (variant, f)
