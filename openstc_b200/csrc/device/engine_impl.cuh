@@ -12,6 +12,7 @@
 #include <string>
 
 #include "engine.hpp"
+#include "face_groups.hpp"
 #include "kernels_mixed.cuh"
 #include "kernels_surrogate.cuh"
 
@@ -949,52 +950,25 @@ class EngineT final : public Engine {
     mark("limit_flow");
   }
 
-  // A box of points that a face kernel reads or writes in a block.
-  struct Touch {
-    int block, lo[3], hi[3];
-    bool meets(const Touch &o) const {
-      if (block != o.block) return false;
-      for (int d = 0; d < 3; ++d)
-        if (hi[d] < o.lo[d] || o.hi[d] < lo[d]) return false;
-      return true;
-    }
-  };
-
-  // Groups faces into launches: a face goes into the launch after the last
-  // earlier face that touches one of its points, so that every pair of faces
-  // whose order could matter keeps it.  order: face indices launch by launch
+  // Faces by launch (face_launch).  order: face indices launch by launch
   // (device), first[l]: the launch's first entry, points[l]: its largest face.
-  // A face's launch lasts 4 to 8 us whatever its size: the mixing layer's 7 faces
-  // take 3 launches (FP64 160 x 96 x 64: 79 -> 51 us).
   struct FaceLaunches {
     int *order = nullptr;
     std::vector<int> first, points;
   };
 
-  FaceLaunches group_faces(const std::vector<std::vector<Touch>> &touch, const std::vector<int> &points) {
-    const int n = static_cast<int>(touch.size());
-    std::vector<int> level(n, 0);
-    int levels = 0;
-    for (int q = 0; q < n; ++q) {
-      if (points[q] <= 0) continue;
-      for (int e = 0; e < q; ++e) {
-        if (points[e] <= 0) continue;
-        bool meet = false;
-        for (const Touch &x : touch[q])
-          for (const Touch &y : touch[e]) meet = meet || x.meets(y);
-        if (meet) level[q] = std::max(level[q], level[e] + 1);
-      }
-      levels = std::max(levels, level[q] + 1);
-    }
+  FaceLaunches group_faces(const std::vector<FacePoints> &faces) {
+    const std::vector<int> launch = face_launch(faces);
+    const int levels = launch.empty() ? 0 : *std::max_element(launch.begin(), launch.end()) + 1;
     FaceLaunches g;
     std::vector<int> order;
     for (int l = 0; l < levels; ++l) {
       g.first.push_back(static_cast<int>(order.size()));
       g.points.push_back(0);
-      for (int q = 0; q < n; ++q)
-        if (points[q] > 0 && level[q] == l) {
+      for (int q = 0; q < static_cast<int>(faces.size()); ++q)
+        if (launch[q] == l) {
           order.push_back(q);
-          g.points[l] = std::max(g.points[l], points[q]);
+          g.points[l] = std::max(g.points[l], faces[q].points);
         }
     }
     g.first.push_back(static_cast<int>(order.size()));
@@ -1010,47 +984,16 @@ class EngineT final : public Engine {
     return g;
   }
 
-  // k_bc touches ngg layers on both sides of its face
   void group_bcs() {
-    std::vector<std::vector<Touch>> touch;
-    std::vector<int> points;
-    for (const HostBc &f : setup_.bcs) {
-      Touch t{f.block, {f.start[0], f.start[1], f.start[2]}, {f.end[0], f.end[1], f.end[2]}};
-      t.lo[f.face] -= setup_.ngg;
-      t.hi[f.face] += setup_.ngg;
-      touch.push_back({t});
-      points.push_back((f.end[0] - f.start[0] + 1) * (f.end[1] - f.start[1] + 1) * (f.end[2] - f.start[2] + 1));
-    }
-    bc_launches_ = group_faces(touch, points);
+    std::vector<FacePoints> faces;
+    for (const HostBc &f : setup_.bcs) faces.push_back(face_points(f, setup_.ngg));
+    bc_launches_ = group_faces(faces);
   }
 
-  // k_inner touches its own points (plane and ghosts, with exact faces also the
-  // tangential ghost rows) and the points they map to in the other block
   void group_inner() {
-    std::vector<std::vector<Touch>> touch;
-    std::vector<int> points;
-    const int tg = setup_.exact_inner ? setup_.ngg : 0;
-    for (const HostInner &f : setup_.inner) {
-      Touch own{f.block, {}, {}}, other{f.target_block, {}, {}};
-      int lo[3], hi[3], np = 1;  // range of d = loop_dir * n
-      for (int q = 0; q < 3; ++q) {
-        const int wide = q != f.face && f.n_point[q] > 1 ? tg : 0;
-        const int e0 = f.loop_dir[q] * -wide, e1 = f.loop_dir[q] * (f.n_point[q] - 1 + wide);
-        lo[q] = std::min(e0, e1);
-        hi[q] = std::max(e0, e1);
-        own.lo[q] = f.start[q] + lo[q];
-        own.hi[q] = f.start[q] + hi[q];
-        np *= f.n_point[q] + 2 * wide;
-      }
-      for (int q = 0; q < 3; ++q) {
-        const int e0 = f.tstart[q] + f.tloop_dir[q] * lo[f.src_tar[q]], e1 = f.tstart[q] + f.tloop_dir[q] * hi[f.src_tar[q]];
-        other.lo[q] = std::min(e0, e1);
-        other.hi[q] = std::max(e0, e1);
-      }
-      touch.push_back({own, other});
-      points.push_back(f.n_point[0] * f.n_point[1] * f.n_point[2] > 0 ? np : 0);
-    }
-    inner_launches_ = group_faces(touch, points);
+    std::vector<FacePoints> faces;
+    for (const HostInner &f : setup_.inner) faces.push_back(face_points(f, setup_.exact_inner ? setup_.ngg : 0));
+    inner_launches_ = group_faces(faces);
   }
 
   void launch_bcs() {
