@@ -80,13 +80,14 @@ struct DevBlock {
   unsigned char *lu_piv;
   double *dq, *dq0, *dqk, *inv_spec, *visc_spec, *dt_local, *bv_last;
   // DPLUR, layout D (FP64 path): the species enthalpies h_k(T) of each cell
-  // (k_dq0) and the terms of its flux-Jacobian product that no direction
-  // enters (sweep_terms): [0] the total enthalpy, [1 + 2 s], [2 + 2 s] the
-  // pressure terms of the increments in buffer s (0 dq, 1 dq0, 2 dqk)
+  // and the terms of its flux-Jacobian product that no direction enters: [0] the
+  // total enthalpy, [1 + 2 s], [2 + 2 s] the pressure terms of the increments in
+  // buffer s (0 dq, 1 dq0, 2 dqk).  k_sweep_terms writes them for dq0, each
+  // sweep the pressure terms of its own increments.
   double *h_spec, *terms;
   // the same on the FP32-bulk path: the weights of the species increments in
-  // the pressure term (ns components, k_dq0), the pressure term of dqf[s]
-  // ([s]), and the inviscid spectral radii with the total enthalpy (k_dq0)
+  // the pressure term (ns components), the pressure term of dqf[s] ([s]), and
+  // the inviscid spectral radii with the total enthalpy
   float *weight32, *terms32;
   float4 *radii32;
   // chemistry surrogate (layout Z; null when off): cells the surrogate judged

@@ -88,8 +88,17 @@ class EngineT final : public Engine {
                  "copy wall");
     }
     source_smem_ = C::mix == 2 ? 2 * std::max(1, s.params.nr) * kCta * sizeof(double) : 0;
-    flux_smem_ = C::nv * kCta * (C::mixed ? sizeof(float) : sizeof(double));
-    col_smem_ = sizeof(double) * ColSmem<C::nv>::size;
+    if constexpr (!C::mixed) {
+      flux_smem_ = C::nv * kCta * sizeof(double);
+      col_smem_ = sizeof(double) * ColSmem<C::nv>::size;
+      if (col_smem_ > 48 * 1024)
+        cuda_check(cudaFuncSetAttribute(k_flux_col<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(col_smem_)),
+                   "column flux smem");
+      if (row_smem<C>() > 48 * 1024)
+        cuda_check(cudaFuncSetAttribute(k_flux_row<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, row_smem<C>()),
+                   "row flux smem");
+    }
     // the EPI matrix, a slice per thread
     dq0_smem_ = 0;
     if (C::mix == 2 && s.params.chem_src_method == 1) {
@@ -100,15 +109,6 @@ class EngineT final : public Engine {
       cuda_check(cudaFuncSetAttribute(k_dq0<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(dq0_smem_)),
                  "dq0 smem");
-    if (col_smem_ > 48 * 1024)
-      cuda_check(cudaFuncSetAttribute(k_flux_col<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(col_smem_)),
-                 "column flux smem");
-    if constexpr (!C::mixed) {
-      if (row_smem<C>() > 48 * 1024)
-        cuda_check(cudaFuncSetAttribute(k_flux_row<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, row_smem<C>()),
-                   "row flux smem");
-    }
     if (source_smem_ > 48 * 1024) {
       if constexpr (C::mixed) {
         cuda_check(cudaFuncSetAttribute(source_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,

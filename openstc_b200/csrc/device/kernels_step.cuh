@@ -1429,8 +1429,8 @@ __global__ void k_inner(const DevBlock *__restrict__ blks, const DevInner *__res
 // Exact inner faces: the first ghost layer of an array that the stencils
 // read across the face, copied from the neighbour's interior (the point map
 // of k_inner).  set: 0 mu_t and lambda_t, 1 |V|, 2 the inviscid spectral
-// radii, 3 the DPLUR increments of buffer dq_sel (0 dq, 1 dq0, 2 dqk), 4 the
-// species enthalpies of the sweeps.
+// radii, 3 the DPLUR increments of buffer dq_sel (0 dq, 1 dq0, 2 dqk) and
+// their pressure terms, 4 the total enthalpy of the sweeps.
 enum HaloSet { kHaloTurb = 0, kHaloVel = 1, kHaloSpec = 2, kHaloDq = 3, kHaloEnthalpy = 4 };
 
 template <class C>

@@ -1,6 +1,6 @@
 // Chemistry surrogate: data generation with the FP64 EPI step, training with
-// the tcgen05 BF16 GEMM, fused tensor-core inference behind a trust gate,
-// and the C-ABI entry points.
+// the tcgen05 layer kernels of mlp_train.cuh, the plain BF16 GEMM, and the host
+// side of the fused tensor-core inference behind a trust gate.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -93,7 +93,6 @@ __device__ inline double gauss(uint64_t &s) {
 }
 
 __device__ inline uint16_t bf16(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
-__device__ inline float from_bf16(uint16_t v) { return __bfloat162float(__ushort_as_bfloat16(v)); }
 
 // ------------------------------------------------------------------ samples
 // T, p, Y[9], dt per sample: from the cells of a flow field (perturbed) or

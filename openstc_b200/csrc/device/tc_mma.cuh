@@ -1,8 +1,8 @@
 // Fifth-generation tensor-core (tcgen05) building blocks for sm_100a:
 // tensor-memory allocation, shared-memory matrix descriptors, BF16 MMA with
 // FP32 accumulation in tensor memory, commit to an mbarrier, and loads of the
-// accumulator back to registers.  Used by the chemistry-surrogate training
-// GEMM and the fused inference kernel.
+// accumulator back to registers.  Used by the chemistry surrogate's
+// training and inference kernels and by the plain BF16 GEMM.
 //
 // Operand tiles live in shared memory in the K-major, no-swizzle canonical
 // layout: 8-row x 16-byte core matrices (8 rows of 8 bf16 along K, 128 bytes,
