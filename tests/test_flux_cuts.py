@@ -1,6 +1,7 @@
 """The cost rule of the flux launches (csrc/device/flux_cut.hpp)."""
 import pytest
 
+from config_cases import FORM_GRIDS
 from flux_cuts import FP64_GRIDS, MIXED_GRIDS, fp64_cut, march_cut
 
 
@@ -12,6 +13,9 @@ def test_the_grids_of_the_gpu_tests_take_every_cut():
     for q in range(2):  # y, z
         assert {m[q] for cuts in MIXED_GRIDS.values() for m in cuts} == {1, 2, 4, 8, 16}
     assert [fp64_cut((n, n // 2, 1), air=True) for n in (48, 256)] == ["rows", 1]
+    # every model: rows in 3-D for air, rows and columns of three lengths for mixtures, both in 2-D
+    assert [fp64_cut(g) for g in FORM_GRIDS] == ["rows", 1, 2, 8, "rows", 1]
+    assert [fp64_cut(g, air=True) for g in FORM_GRIDS] == ["rows"] * 5 + [1]
 
 
 def test_the_workloads_take_the_cuts_they_were_measured_with():
