@@ -59,54 +59,68 @@ sys.path.insert(0, str(ROOT / "tests"))
 METRIC = "reacting-RANS Mcell*steps/s: FP32+surrogate vs plain FP64 at 1e-3 rel. L2"
 UNIT = "Mcell*steps/s"
 
-# Algorithmic bytes per cell of each kernel (FP64, 9 species, SST, EPI,
-# DPLUR): every array a kernel needs, counted once per launch.
 # DRAM bytes per cell of one launch, from ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum) on the 128x64x32 case, scaled by cells: the FP64
 # kernels, and the FP32-bulk kernels with every cell's chemistry
-# point-implicit (the surrogate's quiet cells are taken off below).
+# point-implicit (the surrogate's quiet cells are taken off below).  The sweep's
+# is the mean of a step's four.
 KERNEL_TRAFFIC = {
-    "fp64": {"flux": 739.0, "dplur_sweep": 1648.0, "source": 882.0, "dq0": 1504.0},
-    "mixed": {"flux": 708.0, "dplur_sweep": 890.0, "source": 991.0, "dq0": 1107.0},
+    "fp64": {"flux": 699.0, "dplur_sweep": 1415.0, "source": 925.0, "dq0": 1415.0, "sweep_terms": 241.0},
+    "mixed": {"flux_x": 408.0, "flux_y": 476.0, "flux_z": 444.0, "dplur_sweep": 934.0, "source": 730.0, "dq0": 1123.0,
+              "sweep_terms": 197.0},
 }
-# FP32-bulk sweeps, every cell point-implicit (890 B) and with 14.1 % of the
-# cells quiet under the surrogate (801 B): each quiet cell saves 631 B
+# what a cell that is quiet under the surrogate saves an FP32-bulk sweep: the
+# factors and pivots, from captures with none and 14.1 % of the cells quiet
 TRAFFIC_EPI = {"dplur_sweep": 631.0}
 
-# The FP32-bulk path's DPLUR stages, counted the same way: a sweep reads the
-# FP32 copy of its neighbours' state (metric 9, u v w T, gamma, Y and the
-# turbulence scalars 11), the FP32 species enthalpies (9) and spectral radii
-# (3), the input and dq0 increments in FP32 (16 + 16), dt and the SST
-# Jacobian (2) in FP64 and the quiet flag, and writes its FP32 increments
-# (16; the last sweep the FP64 dq, 16 x 8: 80 B per sweep on average); dq0
-# reads dq (16), dt, the radii, T and the SST Jacobian in FP64 and writes dq0
-# in FP32 and the FP32 enthalpies.  EPI_BYTES: what each cell whose chemistry
-# stays point-implicit adds (the surrogate's quiet cells skip it): the sweep
-# reads the EPI factors of the 8 x 8 block (64 FP64) and the pivots (8 B);
-# dq0 reads the EPI Jacobian block and writes the factors and pivots.
+# Algorithmic bytes per cell of each kernel (9 species, SST, EPI, DPLUR): every
+# array a kernel needs, counted once per launch.
+
+# The FP32-bulk path's kernels that read other operands than the FP64 path's,
+# counted the same way; a quad is four FP32 components of a cell.  A sweep reads
+# of its neighbours' state 8 quads (metric 3, rho u v w, Y 2 1/4, the turbulence
+# scalars), the quad of spectral radii and total enthalpy, the pressure term
+# and the increments in FP32 (16), of its own dq0 (16 FP32), dt and the SST
+# Jacobian (1 + 2 FP64) and the quiet flag; it writes FP32 increments and their
+# pressure term from nine weights and a quad with gamma, the last of four
+# sweeps the FP64 dq instead.  dq0 reads dq (16), dt, the radii and the SST
+# Jacobian in FP64 and writes dq0 in FP32; sweep_terms reads dq0, a quad, T,
+# gamma, Y and the radii and writes the nine weights, the quad of radii and the
+# pressure term.  A flux pass reads the 11 quads of its operands and adds to dq.
+# EPI_BYTES: what each cell whose chemistry stays point-implicit adds (the
+# surrogate's quiet cells skip it): the sweep reads the EPI factors of the 8 x 8
+# block (64 FP64) and the pivots (8 B); dq0 reads the EPI Jacobian block and
+# writes the factors and pivots.
 KERNEL_BYTES_MIXED = {
-    "dplur_sweep": 4 * (9 + 4 + 1 + 11) + 4 * 9 + 4 * 3 + 4 * 32 + 8 * (1 + 2) + 80 + 1,
-    "dq0": 8 * (16 + 1 + 3 + 1 + 2) + 4 * 16 + 4 * 9 + 1,
+    "dplur_sweep": (16 * 9 + 4 + 4 * 16) + (4 * 16 + 8 * (1 + 2) + 1) + (3 * (4 * 17 + 4 * 9 + 16) + 8 * 16) / 4,
+    "dq0": 8 * (16 + 1 + 3 + 2) + 4 * 16 + 1,
+    "sweep_terms": (4 * 16 + 16 + 8 * (2 + 9 + 3)) + (4 * 9 + 16 + 4),
+    "flux_x": 16 * 11 + 8 * (32 + 4 + 1),
+    "flux_y": 16 * 11 + 8 * 32,
+    "flux_z": 16 * 11 + 8 * 32,
 }
 EPI_BYTES = {"dplur_sweep": 8 * 64 + 8, "dq0": 2 * 8 * 64 + 8}
 
 KERNEL_BYTES = {
     "source": 8 * (29 + 101),
     "flux": 8 * (59 + 21),
-    # the FP32-bulk flux as one pass per direction: bv 6, sv 11, metric 9, jac,
-    # mu, mu_t, lambda, lambda_t, rho D 9, wall distance read, dq (16) read and
-    # written; the x pass also reads a, gamma and writes the spectral radii
-    # (3 + 1) and dt
-    "flux_x": 8 * (40 + 2 + 32 + 5),
-    "flux_y": 8 * (40 + 32),
-    "flux_z": 8 * (40 + 32),
-    "dq0": 8 * (104 + 106) + 9,
-    "dplur_sweep": 8 * (155 + 16) + 9,
+    # dq 16, the Jacobian 81, dt, the radii 3 and the SST Jacobian 2; dq0, the
+    # factors and pivots
+    "dq0": 8 * (103 + 97) + 9,
+    # dq0 16, u v w |V| T gamma, Y 9; h_k 9 and the three terms
+    "sweep_terms": 8 * (31 + 12),
+    # metric 9, u v w, Y and the turbulence scalars 11, the three terms, radii 3,
+    # increments and dq0 32, dt, factors 81, SST Jacobian 2; three sweeps of four
+    # also |V|, T, gamma and h_k for the two pressure terms they write
+    "dplur_sweep": 8 * (145 + 16 + (12 + 2) * 3 / 4) + 9,
     "update": 8 * (40 + 34),
     "properties": 8 * (11 + 15),
     "limit_flow": 4,
 }
 
+
+# Device memory of a driver per cell of 384x192x64, ghosts included
+FP64_STATE, MIXED_STATE = 1857, 2185
 
 # Tensor-core FLOPs of one cell through the network as the fused kernel runs
 # it (K of the first layer padded to 16, N of the output layer to 16):
@@ -704,7 +718,7 @@ def main() -> None:
         "ms_per_step": ms_max / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": dtype, "data": "synthetic",
         "config": {"workload": workload(size), "path": args.mode, "parallelism": f"replicas x{world}",
-                   "l2": f"inputs larger than L2 (state ~{cells * 1650 / 1e9:.1f} GB)",
+                   "l2": f"inputs larger than L2 (state ~{cells * (FP64_STATE if args.mode == 'fp64' else MIXED_STATE) / 1e9:.1f} GB)",
                    "compared_after_steps": total},
         "accuracy_vs_fp64": {"rel_l2": acc, "bar": 1e-3, "within": all(v <= 1e-3 for v in acc.values())},
         "fp64_ms_per_step": ms_fp64 / K,

@@ -63,8 +63,8 @@ inline double flux_cost(double serial, int ctas, int slots, double a) {
 // Long columns or marches evaluate the fewest faces, short ones keep the SMs
 // of a small grid busy; the constants are from event times on one B200.  FP64
 // (reacting layer, in us; taken before the divisions by constants became
-// products (div_by), which made a full grid 17 % faster: 160 x 96 x 64 is 2.7 ms
-// now; the order is the same):
+// products (div_by), which made a full grid 17 % faster, 160 x 96 x 64 with 4 planes
+// 2.72 ms; the constants were not fitted again):
 //   24 x 16 x 8:    8 / 4 / 2 / 1 planes 652 / 344 / 190 / 112, rows 24
 //   45 x 37 x 21:                        707 / 381 / 225 / 240, rows 217
 //   96 x 64 x 32:                        909 / 872 / 724 / 768, rows 868

@@ -651,9 +651,12 @@ __device__ __forceinline__ void local_time_step_q(const DevBlock &B, const float
 //   y, z: each thread marches over some cells along d, carrying the lower face
 //      from one cell to the next; lanes run along i, the CTA's 4 warps over
 //      the remaining index (k for y, j for z).
-// The variants (flux_cut.hpp) differ in registers: 8 CTAs per SM cap a thread at 64
-// registers, ~400 B of spills.  Measured at 384x192x64 with a march of 8, the three
-// passes take 5.7 ms at 4 CTAs per SM, 5.0 at 6, 4.8 at 7, 4.4 at 8.
+// The variants (flux_cut.hpp) differ in registers: 4, 6 and 8 CTAs per SM cap a thread
+// at 128, 80 and 64 registers, with 60 to 132, 200 to 212 and 292 to 356 B of spill
+// stores.  The loads in flight decide all the same: the three passes take 4.08, 3.52
+// and 3.17 ms at 384x192x64, 1.02, 0.89 and 0.74 ms at 160x96x64 (one B200), and with a
+// march of 16 instead of 8 at 8 CTAs 3.09 and 0.74 ms.
+
 __device__ __forceinline__ void dir_tile(const Tiles &T, int &b, int &t0, int &t1, int &t2) {
   int t = tile_of(T, blockIdx.x, b);
   t0 = t % T.ntx[b];
