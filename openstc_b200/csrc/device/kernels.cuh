@@ -177,6 +177,26 @@ __device__ __forceinline__ double ipow(double c, int e) {
   return e == 1 ? c : (e == 2 ? c * c : (e == 3 ? c * c * c : std::pow(c, e)));
 }
 
+// chemical_source, src/FiniteRateChem.cu:155-171: every reaction's terms of
+// every species, those with a coefficient of zero too.
+template <int NS>
+__device__ __forceinline__ void chemical_source(const double *q1, const double *q2, int st, double *omega,
+                                                double *omega_d) {
+  OSTC_UNROLL for (int i = 0; i < NS; ++i) {
+    double creation = 0, od = 0;
+    for (int r = 0; r < cP.nr; ++r) {
+      const double a1 = q1[r * st], a2 = q2[r * st];
+      const int f = cP.sf[r * NS + i], bb = cP.sb[r * NS + i];
+      creation += a2 * f + a1 * bb;
+      od += a1 * f + a2 * bb;
+    }
+    creation *= cP.mw[i] * 1e+3;
+    od *= cP.mw[i] * 1e+3;
+    omega_d[i] = od;
+    omega[i] = creation - od;
+  }
+}
+
 // finite_rate_chemistry, src/FiniteRateChem.cu:7-63 with the rate helpers
 // :65-171.  q1/q2 live in shared memory with stride `st` (CTA size).
 // FAST (the FP32-bulk path, FP64 arithmetic within a few ulps of the
@@ -276,20 +296,7 @@ __device__ __forceinline__ void chemistry(double density, double t, const double
     q1[r * st] = a1;
     q2[r * st] = a2;
   }
-  // chemical_source, src/FiniteRateChem.cu:155-171
-  OSTC_UNROLL for (int i = 0; i < NS; ++i) {
-    double creation = 0, od = 0;
-    for (int r = 0; r < nr; ++r) {
-      const double a1 = q1[r * st], a2 = q2[r * st];
-      const int f = cP.sf[r * NS + i], bb = cP.sb[r * NS + i];
-      creation += a2 * f + a1 * bb;
-      od += a1 * f + a2 * bb;
-    }
-    creation *= cP.mw[i] * 1e+3;
-    od *= cP.mw[i] * 1e+3;
-    omega_d[i] = od;
-    omega[i] = creation - od;
-  }
+  chemical_source<NS>(q1, q2, st, omega, omega_d);
 }
 
 // Calls f(std::integral_constant<int, 0>), ..., f(<N - 1>).
@@ -305,8 +312,10 @@ __device__ __forceinline__ void static_for(F &&f) {
 // zero terms and integer conversions, and (T-dependent only) the powers of
 // p_atm / RT of K_c once per reaction order.  Stored products are rounded
 // (__dmul_rn) as the general form's stores round them.
+// Where a rate is not finite the zero terms count (0 x infinity): the cell
+// takes the general sums, and true is returned.
 template <class M, bool FAST>
-__device__ __forceinline__ void chemistry_fixed(double density, double t, const double *Y, double *omega,
+__device__ __forceinline__ bool chemistry_fixed(double density, double t, const double *Y, double *omega,
                                                 double *omega_d, double *q1, double *q2, int st) {
   constexpr int NS = M::ns;
   const double ln_t = FAST ? std::log(t) : 0.0, t_inv = FAST ? 1.0 / t : 0.0;
@@ -346,6 +355,8 @@ __device__ __forceinline__ void chemistry_fixed(double density, double t, const 
       if constexpr (r == first(1)) pt_p = pow_call(temp_t, cP.order[r]);
     });
   }
+  double zero = 0, zero_g = 0;  // NaN if a rate, a Gibbs energy is not finite
+  OSTC_UNROLL for (int l = 0; l < NS; ++l) zero_g = __fma_rn(g[l], 0.0, zero_g);
   static_for<M::nr>([&](auto rc) {
     constexpr int r = rc, type = M::label[r], order = M::order(r);
     double kf = rate1(r);
@@ -383,7 +394,7 @@ __device__ __forceinline__ void chemistry_fixed(double density, double t, const 
     }
     double kb;
     if constexpr (type != 2) {
-      double d_gibbs = 0;
+      double d_gibbs = zero_g;
       static_for<NS>([&](auto lc) {
         constexpr int l = lc;
         if constexpr (M::nu(r, l) != 0) d_gibbs += g[l] * M::nu(r, l);
@@ -410,9 +421,16 @@ __device__ __forceinline__ void chemistry_fixed(double density, double t, const 
       if constexpr (ef != 0) a1 *= FAST ? ipow(c[j], ef) : (ef == 1 ? pow1[j] : pow2[j]);
       if constexpr (eb != 0) a2 *= FAST ? ipow(c[j], eb) : (eb == 1 ? pow1[j] : pow2[j]);
     });
-    q1[r * st] = __dmul_rn(a1, kf);
-    q2[r * st] = __dmul_rn(a2, kb);
+    a1 = __dmul_rn(a1, kf);
+    a2 = __dmul_rn(a2, kb);
+    q1[r * st] = a1;
+    q2[r * st] = a2;
+    zero = __fma_rn(a1, 0.0, __fma_rn(a2, 0.0, zero));
   });
+  if (zero != 0) {
+    chemical_source<NS>(q1, q2, st, omega, omega_d);
+    return true;
+  }
   static_for<NS>([&](auto ic) {
     constexpr int i = ic;
     double creation = 0, od = 0;
@@ -434,6 +452,7 @@ __device__ __forceinline__ void chemistry_fixed(double density, double t, const 
     omega[i] = __fma_rn(creation, w, -od);  // as the general form contracts
     omega_d[i] = od;
   });
+  return false;
 }
 
 // Row m of the same sum for a run-time mechanism: only the reactions that
@@ -449,14 +468,17 @@ __device__ __forceinline__ void jacobian_row(int m, const double *q1, const doub
   }
 }
 
-// M: a compile-time mechanism, or void for the case's own tables.
+// M: a compile-time mechanism, or void for the case's own tables.  True: the
+// Jacobian's rows take the general sums too.
 template <int NS, bool FAST, class M>
-__device__ __forceinline__ void chemistry_of(double density, double t, const double *Y, double *omega, double *omega_d,
+__device__ __forceinline__ bool chemistry_of(double density, double t, const double *Y, double *omega, double *omega_d,
                                              double *q1, double *q2, int st) {
-  if constexpr (std::is_void_v<M>)
+  if constexpr (std::is_void_v<M>) {
     chemistry<NS, FAST>(density, t, Y, omega, omega_d, q1, q2, st);
-  else
-    chemistry_fixed<M, FAST>(density, t, Y, omega, omega_d, q1, q2, st);
+    return true;
+  } else {
+    return chemistry_fixed<M, FAST>(density, t, Y, omega, omega_d, q1, q2, st);
+  }
 }
 
 // Row m of sum_r nu_mr (sf_qr q1_r - sb_qr q2_r), the EPI Jacobian before its
@@ -482,12 +504,34 @@ __device__ __forceinline__ void jacobian_row_fixed(const double *q1, const doubl
   });
 }
 
-template <int NS, class M, int m>
-__device__ __forceinline__ void jacobian_row_of(const double *q1, const double *q2, int st, double *zz) {
-  if constexpr (std::is_void_v<M>)
-    jacobian_row<NS>(m, q1, q2, st, zz);
-  else
-    jacobian_row_fixed<M, m>(q1, q2, st, zz);
+// put(m, zz) for the first `rows` rows of the Jacobian; general: what
+// chemistry_of returned.
+template <int NS, class M, class Put>
+__device__ __forceinline__ void jacobian_rows(bool general, int rows, const double *q1, const double *q2, int st,
+                                              Put &&put) {
+  if constexpr (std::is_void_v<M>) {
+    static_for<NS>([&](auto mc) {
+      constexpr int m = mc;
+      if (m >= rows) return;
+      double zz[NS];
+      jacobian_row<NS>(m, q1, q2, st, zz);
+      put(m, zz);
+    });
+  } else if (!general) {
+    static_for<NS>([&](auto mc) {
+      constexpr int m = mc;
+      if (m >= rows) return;
+      double zz[NS];
+      jacobian_row_fixed<M, m>(q1, q2, st, zz);
+      put(m, zz);
+    });
+  } else {
+    _Pragma("unroll 1") for (int m = 0; m < rows; ++m) {
+      double zz[NS];
+      jacobian_row<NS>(m, q1, q2, st, zz);
+      put(m, zz);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- inviscid

@@ -485,7 +485,7 @@ __device__ __forceinline__ void chem_cell(const DevBlock &B, int64_t n, int64_t 
   double Y[NS], omega[NS], omega_d[NS];
   OSTC_UNROLL for (int l = 0; l < NS; ++l) Y[l] = ld(B.sv + l * sz + n);
   const double density = ld(B.bv + n), t = ld(B.bv + 5 * sz + n);
-  chemistry_of<NS, true, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
+  const bool general = chemistry_of<NS, true, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
   const double jac = ld(B.jac + n);
   OSTC_UNROLL for (int l = 0; l < NS; ++l) dq_spec[l] = jac * omega[l];
   const int method = cP.chem_src_method;
@@ -497,11 +497,7 @@ __device__ __forceinline__ void chem_cell(const DevBlock &B, int64_t n, int64_t 
     double inv_rho_y[NS];
     OSTC_UNROLL for (int q = 0; q < NS; ++q) inv_rho_y[q] = Y[q] > 1e-25 ? 1.0 / (density * Y[q]) : 0.0;
     // only the leading na x na block (the other rows and columns are zero)
-    static_for<NS>([&](auto mc) {
-      constexpr int m = mc;
-      if (m >= na) return;
-      double zz[NS];
-      jacobian_row_of<NS, M, m>(q1, q2, kCta, zz);
+    jacobian_rows<NS, M>(general, na, q1, q2, kCta, [&](int m, const double *zz) {
       OSTC_UNROLL for (int q = 0; q < NS; ++q) {
         if (q >= na) break;
         const double v = zz[q] * inv_rho_y[q];

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kCta, 4) k_source(const DevBlock *__restrict__
     double Y[NS], omega[NS], omega_d[NS];
     OSTC_UNROLL for (int l = 0; l < NS; ++l) Y[l] = ld(B.sv + l * sz + n);
     const double density = ld(B.bv + n), t = ld(B.bv + 5 * sz + n);
-    chemistry_of<NS, false, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
+    const bool general = chemistry_of<NS, false, M>(density, t, Y, omega, omega_d, q1, q2, kCta);
     const double jac = ld(B.jac + n);
     OSTC_UNROLL for (int l = 0; l < NS; ++l) dq[l + 5] = 0.0 + jac * omega[l];
     const int method = cP.chem_src_method;
@@ -61,10 +61,7 @@ __global__ void __launch_bounds__(kCta, 4) k_source(const DevBlock *__restrict__
       // each row visits only the reactions that change its species (the
       // others add an exact zero in the reference) and sums its terms in
       // reaction order, so the entries are the reference's bit for bit
-      static_for<NS>([&](auto mc) {
-        constexpr int m = mc;
-        double zz[NS];
-        jacobian_row_of<NS, M, m>(q1, q2, kCta, zz);
+      jacobian_rows<NS, M>(general, NS, q1, q2, kCta, [&](int m, const double *zz) {
         OSTC_UNROLL for (int q = 0; q < NS; ++q) {
           const double v = Y[q] > 1e-25 ? zz[q] / (density * Y[q]) : 0.0;
           B.chem_jac[(m * NS + q) * sz0 + nz] = cP.mw[m] * v * 1e+3;

@@ -78,12 +78,9 @@ template <int NS, class M = void>
 __device__ inline void epi_increment(double T, double rho, const double *Y, double dt, double *q1, double *q2,
                                      int stride, double *dy) {
   double omega[NS], omega_d[NS];
-  chemistry_of<NS, false, M>(rho, T, Y, omega, omega_d, q1, q2, stride);
+  const bool general = chemistry_of<NS, false, M>(rho, T, Y, omega, omega_d, q1, q2, stride);
   double lhs[NS * NS];
-  static_for<NS>([&](auto mc) {
-    constexpr int m = mc;
-    double zz[NS];
-    jacobian_row_of<NS, M, m>(q1, q2, stride, zz);
+  jacobian_rows<NS, M>(general, NS, q1, q2, stride, [&](int m, const double *zz) {
     OSTC_UNROLL for (int q = 0; q < NS; ++q) {
       const double v = Y[q] > 1e-25 ? zz[q] / (rho * Y[q]) : 0.0;
       const double J = cP.mw[m] * v * 1e+3;
