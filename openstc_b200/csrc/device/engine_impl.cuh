@@ -688,8 +688,8 @@ class EngineT final : public Engine {
 
   // The chemistry unrolled over the reactions of the shipped mechanism where
   // the case has its stoichiometry, the general loops otherwise.  Source stage
-  // at 160 x 96 x 64, general and unrolled: FP64 2.23 and 1.12 ms, FP32-bulk
-  // path 1.06 and 0.39 ms (one B200).
+  // at 160 x 96 x 64, general and unrolled: FP64 2.12 and 1.11 ms, FP32-bulk
+  // path 1.06 and 0.38 ms (one B200).
   using Fixed = std::conditional_t<C::mix == 2 && C::ns == mech::H2O2::ns, mech::H2O2, void>;
   bool fixed_mechanism() const { return !std::is_void_v<Fixed> && mech::matches<mech::H2O2>(setup_.params); }
 
